@@ -930,7 +930,7 @@ rot_sweep_kernel(const RotArgs a) {
 // The exact (FP64) form of the fused velocity + stretching sum (and of the velocity and PSE
 // sums) with each unordered pair evaluated once for both particles: the pair terms are the
 // FP32 operators' pair2 in double
-// (CUDA's rsqrt(double), as the one-sided FP64 sweep), and they differ from the one-sided
+// (rsqrt_fp64, as the one-sided FP64 sweep), and they differ from the one-sided
 // sweep's only in rounding (the triple product a_i . (r x a_j) in place of
 // r . ((a_j - a_i) x a_i)); the sums are FP64 throughout, so there are no windows and no
 // carries: each lane keeps R = 2 kP targets' sums in registers, and the source's sums travel
