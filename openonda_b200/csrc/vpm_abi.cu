@@ -23,6 +23,7 @@
 #include "vpm_sweep.cuh"
 #include "vpm_adjoint.cuh"
 #include "vpm_rot.cuh"
+#include "vpm_scalar.cuh"
 
 namespace vpm {
 namespace {
@@ -95,6 +96,7 @@ struct Plan {
   // both-sides sweep: the diagonal tiles run beside the (single) diagonal-pair launch on a
   // second stream, into their own accumulator sets after the pairs' ones
   int diag_beside = 0;
+  int scalar = 0;  // FP64 scalar diagnostics with each unordered pair once (vpm_scalar.cuh)
 };
 
 // FP32 self sums with at least this many particles evaluate each unordered pair once for both
@@ -709,6 +711,94 @@ struct RotSweep {
   }
 };
 
+// FP64 scalar diagnostics over all particles (vpm_scalar.cuh): launch plan and launches.
+template <class Op>
+struct ScalarSweep {
+  template <int R>
+  static const void* kernel() {
+    return reinterpret_cast<const void*>(&scalar_pairs_kernel<Op, R>);
+  }
+
+  template <int R>
+  static int occupancy(int* occ) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    const auto key = std::make_pair(kernel<R>(), dev);
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_occ.find(key);
+    if (it == g_occ.end()) {
+      int o = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kernel<R>(), kScalarThreads, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+      it = g_occ.emplace(key, o > 0 ? o : 1).first;
+    }
+    *occ = it->second;
+    return VPM_OK;
+  }
+
+  // Splits of a target tile's source list: the count whose waves of equal blocks take the least
+  // time, a block costing its pieces and about one more for its start and reduction.
+  template <int R>
+  static double best_splits(int64_t n, int64_t slots, Plan* p) {
+    const int64_t T = int64_t(kScalarThreads) * R;
+    const int64_t nt = (n + T - 1) / T;
+    const int64_t pieces = (1 + nt / 2) * (T / kScalarPiece);
+    double best = -1.0;
+    for (int64_t s = 1; s <= 256 && s <= pieces; ++s) {
+      const int64_t chunk = (pieces + s - 1) / s;
+      const int64_t se = (pieces + chunk - 1) / chunk;
+      if (se != s) continue;
+      const double waves = std::ceil(double(nt * se) / double(slots));
+      const double cost = waves * (double(chunk) + 1.0) * R;
+      if (best < 0.0 || cost < best) {
+        best = cost;
+        p->splits = int(se);
+        p->chunk = chunk;
+      }
+    }
+    p->tblocks = nt;
+    p->threads = kScalarThreads;
+    p->r = R;
+    p->nv = 1;
+    p->scalar = 1;
+    return best;
+  }
+
+  static int plan(int64_t n, Plan* p) {
+    DevInfo d;
+    int rc = device_info(&d);
+    int o1 = 1, o2 = 1;
+    if (!rc) rc = occupancy<1>(&o1);
+    if (!rc) rc = occupancy<2>(&o2);
+    if (rc) return rc;
+    Plan p1, p2;
+    // work per SM and piece is R x the resident blocks; the cheaper of the two builds
+    const double c1 = best_splits<1>(n, int64_t(d.sms) * o1, &p1) * o1;
+    const double c2 = best_splits<2>(n, int64_t(d.sms) * o2, &p2) * o2;
+    *p = c1 < c2 ? p1 : p2;
+    return VPM_OK;
+  }
+
+  // partial: [p.splits][p.tblocks][2], within the plan's p.splits * n doubles (n > 1; one tile's
+  // two doubles fit the region's alignment)
+  static int launch(const Plan& p, const Rec<double>* rec, int64_t n, double* partial,
+                    double scale, double* out, cudaStream_t st) {
+    const ScalarArgs a{rec, n, int(p.tblocks), int(p.chunk), partial};
+    const dim3 grid(unsigned(p.tblocks), unsigned(p.splits));
+    if (p.r == 1)
+      scalar_pairs_kernel<Op, 1><<<grid, kScalarThreads, 0, st>>>(a);
+    else
+      scalar_pairs_kernel<Op, 2><<<grid, kScalarThreads, 0, st>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "scalar sweep launch");
+    // each unordered pair was counted once
+    scalar_total_kernel<<<1, 1024, 0, st>>>(partial, int(p.tblocks) * p.splits, 2.0 * scale, out);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? VPM_OK : cuda_fail(e, "reduce launch");
+  }
+};
+
 // ---- adjoint: pack, finalize --------------------------------------------------------------
 template <class E>
 __global__ void pack_grad_kernel(const double* __restrict__ pos, const double* __restrict__ str,
@@ -844,6 +934,9 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
       }
       return Sweep<typename O::Vel, T>::plan(m, n, p, mpb);
     case VPM_OP_TOTAL_HELICITY:
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (m == n && n > 0) return ScalarSweep<ScalarHel>::plan(n, p);
+      }
       return Sweep<typename O::Vel, T>::plan(m, n, p, mpb);
     case VPM_OP_INDUCED_VELOCITY_AT:
       return Sweep<typename O::VelAt, T>::plan(m, n, p, mpb);
@@ -861,8 +954,14 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
       }
       return Sweep<typename O::Pse, T>::plan(m, n, p, mpb);
     case VPM_OP_TOTAL_KINETIC_ENERGY:
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (m == n && n > 0) return ScalarSweep<ScalarKe>::plan(n, p);
+      }
       return Sweep<typename O::Ke, T>::plan(m, n, p, mpb);
     case VPM_OP_TOTAL_ENSTROPHY:
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (m == n && n > 0) return ScalarSweep<ScalarEns>::plan(n, p);
+      }
       return Sweep<typename O::Ens, T>::plan(m, n, p, mpb);
     case VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
@@ -1131,6 +1230,19 @@ int run(const Call& c) {
     case VPM_OP_TOTAL_HELICITY:
     case VPM_OP_TOTAL_ENSTROPHY: {
       double scale = 0.0;
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (p.scalar) {
+          const double extra = c.ref_extra_4pi ? 4.0 * kPi : 1.0;
+          if (c.op == VPM_OP_TOTAL_KINETIC_ENERGY)
+            return ScalarSweep<ScalarKe>::launch(p, src, c.n, part, 1.0 / (16.0 * kPi), c.out,
+                                                 c.st);
+          if (c.op == VPM_OP_TOTAL_HELICITY)
+            return ScalarSweep<ScalarHel>::launch(p, src, c.n, part, -1.0 / (4.0 * kPi) / extra,
+                                                  c.out, c.st);
+          return ScalarSweep<ScalarEns>::launch(p, src, c.n, part, 1.0 / (8.0 * kPi) / extra,
+                                                c.out, c.st);
+        }
+      }
       if (c.op == VPM_OP_TOTAL_KINETIC_ENERGY) {
         rc = Sweep<typename O::Ke, T>::launch(p, tgt, c.m, c.tgt_begin, src, c.n, part, c.st);
         scale = 1.0 / (16.0 * kPi);
