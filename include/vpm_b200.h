@@ -170,7 +170,8 @@ int vpm_velocity_and_strength_gradients(const double* positions, const double* s
  * (default 24576).  No counterpart in the reference. */
 int64_t vpm_set_symmetric_min_n(int64_t n);
 /* Kernel launches of one sweep of `op` (sweep and finalize, not the packing of the inputs)
- * for m targets and n sources under the current plan; -1 on error. */
+ * for m targets and n sources under the current plan; -1 on error.  1: a small sum, whose one
+ * launch also packs the caller's arrays (from packed records it takes sweep and finalize). */
 int64_t vpm_sweep_launches(int op, int precision, int64_t m, int64_t n);
 
 /* The four pair sums of one dynamic-LES time step on the same state, in one sweep:

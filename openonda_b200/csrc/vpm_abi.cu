@@ -24,6 +24,7 @@
 #include "vpm_adjoint.cuh"
 #include "vpm_rot.cuh"
 #include "vpm_scalar.cuh"
+#include "vpm_small.cuh"
 
 namespace vpm {
 namespace {
@@ -96,6 +97,7 @@ struct Plan {
   // both-sides sweep: the diagonal tiles run beside the (single) diagonal-pair launch on a
   // second stream, into their own accumulator sets after the pairs' ones
   int diag_beside = 0;
+  int small = 0;   // one launch from the caller's arrays (vpm_small.cuh); records: one-sided
   int scalar = 0;  // FP64 scalar diagnostics with each unordered pair once (vpm_scalar.cuh)
 };
 
@@ -887,6 +889,107 @@ __global__ void finalize_kegrad_kernel(const double* __restrict__ part, int spli
   gsig[i] = 0.5 * c * v[6];
 }
 
+// ---- small sums in one launch (vpm_small.cuh) ---------------------------------------------
+// Taken for a vector sum from the caller's arrays with fewer than kSmallSources sources (four
+// windows per warp of the largest cluster) and at most small_pairs pairs.  Measured against the
+// three launches (us, self sums): FP64 velocity 15.0 / 27 at 2000 and 28.2 / 26.1 at 3000
+// particles, fused 20.2 / 37 and 39.6 / 39.1; FP32c velocity 9.1 / 24 at 2000, 14.8 / 16.8 at 3000
+// and 22.3 / 25.3 at 4000, fused 13.5 / 45, 22.0 / 29.4 and 34.7 / 41.1.
+constexpr int64_t kSmallSources = 4096;
+template <class T>
+constexpr int64_t small_pairs = LaneTraits<T>::kLanes == 1 ? 6000000 : 16000000;
+
+int64_t small_windows(int64_t n) { return (n + kSmallWindow - 1) / kSmallWindow; }
+
+template <class T>
+bool small_usable(int64_t m, int64_t n) {
+  return m > 0 && n > 0 && n < kSmallSources && m <= small_pairs<T> / n;
+}
+
+template <class T, int KIND, int NV>
+struct SmallFinalize {
+  __device__ __forceinline__ static void write(const double (&v)[NV], const Rec<T>* rec,
+                                               double* out, double* out2) {
+    finalize_values<T, KIND, NV>(v, rec, 0, out, out2, nullptr);
+  }
+};
+
+template <class Op, class T, int KIND>
+struct SmallSweep {
+  static constexpr int R = LaneTraits<T>::kLanes;  // one lane of targets per thread
+  static constexpr auto kKernel =
+      &small_sweep_kernel<Op, T, R, SmallFinalize<T, KIND, Op::NV>>;
+
+  // Resident blocks per SM (asked for when the plan is made: the query also loads the kernel,
+  // so that a stream capture after it only launches).
+  static int prepare(int* occ) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    const auto key = std::make_pair(reinterpret_cast<const void*>(kKernel), dev);
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_occ.find(key);
+    if (it == g_occ.end()) {
+      int o = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kKernel, kSmallThreads, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+      it = g_occ.emplace(key, o > 0 ? o : 1).first;
+    }
+    *occ = it->second;
+    return VPM_OK;
+  }
+
+  static int launch(SmallArgs a, cudaStream_t st) {
+    DevInfo d;
+    int occ = 1;
+    int rc = device_info(&d);
+    if (!rc) rc = prepare(&occ);
+    if (rc) return rc;
+    // cluster size: the one whose waves of resident blocks walk the fewest windows; a larger
+    // cluster costs about a sixteenth of a window more for its reduction
+    const double slots = double(d.sms) * (occ < 4 ? occ : 4);
+    const int64_t tiles = (int64_t(a.m) + 32 * R - 1) / (32 * R);
+    const int64_t windows = small_windows(a.n);
+    int S = 1;
+    double best = -1.0;
+    for (int s = 1; s <= kSmallMaxCluster; s *= 2) {
+      const int64_t per = (windows + kSmallWarps * s - 1) / (kSmallWarps * s);
+      const double waves = std::ceil(double(tiles * s) / slots);
+      const double cost = waves * (double(per) + 0.25) + s / 16.0;
+      if (best < 0.0 || cost < best) {
+        best = cost;
+        S = s;
+        a.windows_per_warp = int(per);
+      }
+  }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(tiles * S));
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(S);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kKernel, a);
+    return e == cudaSuccess ? VPM_OK : cuda_fail(e, "small sweep launch");
+  }
+};
+
+// The one-sided plan of a vector sum; small sums from the caller's arrays take one launch.
+template <class Op, class T, int KIND>
+int plan_vector(int64_t m, int64_t n, Plan* p, size_t mpb) {
+  int rc = Sweep<Op, T>::plan(m, n, p, mpb);
+  if (!rc && small_usable<T>(m, n)) {
+    int occ = 0;
+    rc = SmallSweep<Op, T, KIND>::prepare(&occ);
+    p->small = 1;
+  }
+  return rc;
+}
+
 // ---- operator selection -----------------------------------------------------------------
 // UC: all cores equal (VPM_UNIFORM_CORE); the probe sums and the kinetic energy keep the
 // general form.
@@ -932,18 +1035,18 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
         if (RotSweep<typename O::VelBoth64>::usable(m, n, mpb))
           return RotSweep<typename O::VelBoth64>::plan(n, p, mpb);
       }
-      return Sweep<typename O::Vel, T>::plan(m, n, p, mpb);
+      return plan_vector<typename O::Vel, T, FIN_VEL>(m, n, p, mpb);
     case VPM_OP_TOTAL_HELICITY:
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarHel>::plan(n, p);
       }
       return Sweep<typename O::Vel, T>::plan(m, n, p, mpb);
     case VPM_OP_INDUCED_VELOCITY_AT:
-      return Sweep<typename O::VelAt, T>::plan(m, n, p, mpb);
+      return plan_vector<typename O::VelAt, T, FIN_VEL>(m, n, p, mpb);
     case VPM_OP_VORTICITY_FIELD_AT:
-      return Sweep<typename O::VortAt, T>::plan(m, n, p, mpb);
+      return plan_vector<typename O::VortAt, T, FIN_VORT>(m, n, p, mpb);
     case VPM_OP_STRENGTH_GRADIENTS:
-      return Sweep<typename O::Stretch, T>::plan(m, n, p, mpb);
+      return plan_vector<typename O::Stretch, T, FIN_STRETCH>(m, n, p, mpb);
     case VPM_OP_STRENGTH_GRADIENTS_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::PseBoth>::usable(m, n, mpb))
@@ -952,7 +1055,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
         if (RotSweep<typename O::PseBoth64>::usable(m, n, mpb))
           return RotSweep<typename O::PseBoth64>::plan(n, p, mpb);
       }
-      return Sweep<typename O::Pse, T>::plan(m, n, p, mpb);
+      return plan_vector<typename O::Pse, T, FIN_PSE>(m, n, p, mpb);
     case VPM_OP_TOTAL_KINETIC_ENERGY:
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarKe>::plan(n, p);
@@ -1001,7 +1104,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
         if (RotSweep<typename O::VelStretchBoth64>::usable(m, n, mpb))
           return RotSweep<typename O::VelStretchBoth64>::plan(n, p, mpb);
       }
-      return Sweep<typename O::VelStretch, T>::plan(m, n, p, mpb);
+      return plan_vector<typename O::VelStretch, T, FIN_VELSTRETCH>(m, n, p, mpb);
     case VPM_OP_LES_STEP_SUMS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::LesStepBoth>::usable(m, n, mpb))
@@ -1119,6 +1222,28 @@ int run(const Call& c) {
   if (c.ws_bytes < L.total)
     return fail(VPM_ERR_WORKSPACE, "workspace has " + std::to_string(c.ws_bytes) +
                                        " bytes, needs " + std::to_string(L.total));
+  if (p.small && !c.records) {
+    const bool probe = is_probe(c.op);
+    const SmallArgs a{probe ? c.tgt : c.pos, probe ? nullptr : c.str, c.nu,     c.pos,
+                      c.str,                 c.rad,                   int(c.m), int(c.n),
+                      1,                     int(UC),                 c.out,    c.out2};
+    switch (c.op) {
+      case VPM_OP_SELFINDUCED_VELOCITY:
+        return SmallSweep<typename O::Vel, T, FIN_VEL>::launch(a, c.st);
+      case VPM_OP_INDUCED_VELOCITY_AT:
+        return SmallSweep<typename O::VelAt, T, FIN_VEL>::launch(a, c.st);
+      case VPM_OP_VORTICITY_FIELD_AT:
+        return SmallSweep<typename O::VortAt, T, FIN_VORT>::launch(a, c.st);
+      case VPM_OP_STRENGTH_GRADIENTS:
+        return SmallSweep<typename O::Stretch, T, FIN_STRETCH>::launch(a, c.st);
+      case VPM_OP_STRENGTH_GRADIENTS_PSE:
+        return SmallSweep<typename O::Pse, T, FIN_PSE>::launch(a, c.st);
+      case VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS:
+        return SmallSweep<typename O::VelStretch, T, FIN_VELSTRETCH>::launch(a, c.st);
+      default:
+        break;
+    }
+  }
   char* ws = static_cast<char*>(c.ws);
   Rec<T>* src = c.records ? const_cast<Rec<T>*>(static_cast<const Rec<T>*>(c.records))
                           : reinterpret_cast<Rec<T>*>(ws + L.src_off);
@@ -1918,6 +2043,7 @@ int64_t vpm_sweep_launches(int op, int precision, int64_t m, int64_t n) {
     const int64_t npairs = p.tblocks / 2;
     return 3 + (npairs + p.pairs - 1) / p.pairs;
   }
+  if (p.small) return 1;  // pack, sweep and finalize in one
   return 2;  // sweep, finalize (or the single-block reduction of a scalar)
 }
 

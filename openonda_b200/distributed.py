@@ -189,9 +189,10 @@ class ShardedVelocityStretching:
             self.ws_bytes = kernels.workspace_bytes("velocity_and_strength_gradients",
                                                     precision, self.m, self.n)
             # the sweep's own launches (one-sided: sweep + finalize; both-sides sweep over all
-            # particles: zero, diagonal tiles, diagonal-pair launches, finalize)
-            self.sweep_launches = int(lib.vpm_sweep_launches(
-                _lib.OPS["velocity_and_strength_gradients"], self.pcode, self.m, self.n))
+            # particles: zero, diagonal tiles, diagonal-pair launches, finalize); the one launch
+            # of small sums reads arrays, not records
+            self.sweep_launches = max(2, int(lib.vpm_sweep_launches(
+                _lib.OPS["velocity_and_strength_gradients"], self.pcode, self.m, self.n)))
             self.both_sides = self.sweep_launches > 2
         self.ws = torch.empty(max(self.ws_bytes, 256), dtype=torch.uint8, device=dev)
         self.kernel_launches_per_call = 1 + self.sweep_launches  # + the pack

@@ -254,7 +254,8 @@ def set_symmetric_min_n(n: int) -> int:
 
 
 def sweep_launches(op: str, precision: str, m: int, n: int, uniform_core: bool = False) -> int:
-    """Kernel launches of one sweep of ``op`` (sweep and finalize) under the current plan."""
+    """Kernel launches of one sweep of ``op`` (sweep and finalize; 1 for a small sum, packing
+    included) under the current plan."""
     v = int(_lib.load().vpm_sweep_launches(_lib.OPS[op],
                                            _lib.precision_code(precision, uniform_core),
                                            int(m), int(n)))
