@@ -166,8 +166,11 @@ int vpm_velocity_and_strength_gradients(const double* positions, const double* s
  * particles), the diagonal tiles run on a second stream of the library's, forked from and
  * joined to the caller's stream by events inside the call, so stream order and CUDA-graph
  * capture see one call as before; that stream is created by the first such call in a context
- * (make it before any stream capture).  Sets the threshold and returns the previous one
- * (default 24576).  No counterpart in the reference. */
+ * (make it before any stream capture).  The FP64 self sums (those above, the stretching and
+ * the adjoint among them) do so from a sixth of this value on, in one launch over a circle of
+ * tiles; the stretching and the adjoint stay there while their partial sums fit 4 GB.  The scalar
+ * diagnostics in FP64 take each unordered pair once at every size.  Sets the threshold and
+ * returns the previous one (default 24576).  No counterpart in the reference. */
 int64_t vpm_set_symmetric_min_n(int64_t n);
 /* Kernel launches of one sweep of `op` (sweep and finalize, not the packing of the inputs)
  * for m targets and n sources under the current plan; -1 on error.  1: a small sum, whose one

@@ -23,6 +23,8 @@
 #include "vpm_sweep.cuh"
 #include "vpm_adjoint.cuh"
 #include "vpm_rot.cuh"
+#include "vpm_circle.cuh"
+#include "vpm_sets.cuh"
 #include "vpm_scalar.cuh"
 #include "vpm_small.cuh"
 
@@ -76,11 +78,16 @@ struct Cfg<double> {
 #ifndef VPM_MAX_SPLITS
 #define VPM_MAX_SPLITS 64
 #endif
-#ifndef VPM_MIN_CHUNK
-#define VPM_MIN_CHUNK 256
-#endif
 constexpr int kMaxSplits = VPM_MAX_SPLITS;
-constexpr int64_t kMinChunk = VPM_MIN_CHUNK;
+// Shortest split of the sources.  Small sums are bound by the longest chain of sources a thread
+// walks, and with the sets summed by several threads per particle (vpm_sets.cuh) a split more
+// costs little: at 1000 particles chunks of 256 / 64 / 32 took 94 / 27 / 20 us for the FP64
+// adjoint, 85 / 26 / 26 us for the FP64 and 42 / 22 / 24 us for the FP32c LES step sums.
+template <class T>
+constexpr int64_t kMinChunk = LaneTraits<T>::kLanes == 1 ? 32 : 64;
+// The scalar sums' finalize is one block that walks all splits: at 4096 particles and chunks of
+// 64 the FP32c kinetic energy took 74 us, of 256 45 us.
+constexpr int64_t kMinChunkScalar = 256;
 constexpr size_t kMaxPartialBytes = size_t(4) << 30;
 
 struct Plan {
@@ -97,6 +104,8 @@ struct Plan {
   // both-sides sweep: the diagonal tiles run beside the (single) diagonal-pair launch on a
   // second stream, into their own accumulator sets after the pairs' ones
   int diag_beside = 0;
+  Shares shares{};  // of the one-launch schedules
+  int circle = 0;  // FP64 both-sides sweep in one launch (vpm_circle.cuh)
   int small = 0;   // one launch from the caller's arrays (vpm_small.cuh); records: one-sided
   int scalar = 0;  // FP64 scalar diagnostics with each unordered pair once (vpm_scalar.cuh)
 };
@@ -162,7 +171,8 @@ struct Sweep {
     return reinterpret_cast<void*>(&sweep_kernel<Op, T, R, C::THREADS, TILE, C::STAGES, C::MINB>);
   }
 
-  static int plan(int64_t m, int64_t n, Plan* p, size_t max_partial_bytes = kMaxPartialBytes) {
+  static int plan(int64_t m, int64_t n, Plan* p, size_t max_partial_bytes = kMaxPartialBytes,
+                  int64_t min_chunk = kMinChunk<T>) {
     DevInfo d;
     int rc = device_info(&d);
     if (rc) return rc;
@@ -202,7 +212,7 @@ struct Sweep {
     for (int s = 1; s <= kMaxSplits; ++s) {
       int64_t chunk = (n + s - 1) / s;
       chunk = (chunk + kCarryWindow - 1) / kCarryWindow * kCarryWindow;
-      if (s > 1 && chunk < kMinChunk) break;
+      if (s > 1 && chunk < min_chunk) break;
       const int64_t se = (n + chunk - 1) / chunk;
       if (se != s) continue;
       if (size_t(se) * NV * size_t(m) * sizeof(double) > max_partial_bytes) break;
@@ -275,6 +285,11 @@ int pack(const double* pos, const double* str, const double* rad, const double* 
 }
 
 // ---- finalize kernels -----------------------------------------------------------------
+// Splits from which the finalize of a one-sided sweep sums them with kSetLanes threads per
+// particle (vpm_sets.cuh).
+constexpr int kSetLanesMinSplits = 4;
+constexpr int64_t kSetLanesMaxTargets = 1 << 16;
+
 enum FinKind { FIN_VEL = 0, FIN_VORT = 1, FIN_STRETCH = 2, FIN_PSE = 3, FIN_VELSTRETCH = 4,
                FIN_LES = 5 };
 
@@ -333,15 +348,31 @@ __device__ __forceinline__ void finalize_values(const double (&v)[NV], const Rec
   }
 }
 
+// Finalize of finalize_sets_kernel.  scalar (FIN_LES): particle i's enstrophy filter sum, from
+// value 12 (both-sides sums) or from the three components E_i as a_i . E_i (one-sided sums).
+template <class T, int KIND, int NV>
+struct SetsFinalize {
+  const Rec<T>* rec;
+  double *out, *out2, *out3, *scalar;
+  __device__ __forceinline__ void write(const double (&v)[NV], int64_t i) const {
+    finalize_values<T, KIND, NV>(v, rec, i, out, out2, out3);
+    if constexpr (KIND == FIN_LES) {
+      if constexpr (NV == 13)
+        scalar[i] = v[12];
+      else
+        scalar[i] = elem(rec[i].ax) * v[12] + elem(rec[i].ay) * v[13] + elem(rec[i].az) * v[14];
+    }
+  }
+};
+
 template <class T, int KIND, int NV>
 __global__ void finalize_vec_kernel(const double* __restrict__ part, int splits, int64_t m,
-                                    const Rec<T>* __restrict__ tgt, double* __restrict__ out,
-                                    double* __restrict__ out2, double* __restrict__ out3) {
+                                    const SetsFinalize<T, KIND, NV> fin) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= m) return;
   double v[NV];
   sum_splits<NV>(part, splits, m, i, v);
-  finalize_values<T, KIND, NV>(v, tgt, i, out, out2, out3);
+  fin.write(v, i);
 }
 
 // Pair shards across GPUs: rows[i][v] = the sum over the sets s, in order, of acc[s][v][i].
@@ -373,9 +404,9 @@ __global__ void finalize_rows_kernel(const double* __restrict__ rows, int64_t m,
 
 constexpr int kReduceThreads = 1024;
 
-// Single-block, fixed-order reduction of  scale * a_i . V_i  over all targets, V_i being
-// values OFF..OFF+2 of NV partial sums per target.
-template <class T, int NV = 3, int OFF = 0>
+// Single-block, fixed-order reduction of  scale * a_i . V_i  over all targets, V_i being their
+// three sums.
+template <class T>
 __global__ void __launch_bounds__(kReduceThreads)
 finalize_dot_kernel(const double* __restrict__ part, int splits, int64_t m,
                     const Rec<T>* __restrict__ tgt, double scale, double* __restrict__ out) {
@@ -384,7 +415,7 @@ finalize_dot_kernel(const double* __restrict__ part, int splits, int64_t m,
   for (int64_t i = threadIdx.x; i < m; i += kReduceThreads) {
     double v[3] = {0.0, 0.0, 0.0};
     for (int s = 0; s < splits; ++s) {
-      const double* p = part + int64_t(s) * NV * m + int64_t(OFF) * m;
+      const double* p = part + int64_t(s) * 3 * m;
 #pragma unroll
       for (int k = 0; k < 3; ++k) v[k] += p[int64_t(k) * m + i];
     }
@@ -399,19 +430,14 @@ finalize_dot_kernel(const double* __restrict__ part, int splits, int64_t m,
   if (threadIdx.x == 0) out[0] = red[0] * scale;
 }
 
-// scale * the sum over all targets of value OFF of NV partial sums per target, in a fixed
-// order (the same one as finalize_dot_kernel)
-template <int NV, int OFF>
+// scale * the sum of m values, in a fixed order (the same one as finalize_dot_kernel).
 __global__ void __launch_bounds__(kReduceThreads)
-finalize_sum_kernel(const double* __restrict__ part, int splits, int64_t m, double scale,
+finalize_sum_kernel(const double* __restrict__ v, int64_t m, double scale,
                     double* __restrict__ out) {
   __shared__ double red[kReduceThreads];
   double acc = 0.0;
-  for (int64_t i = threadIdx.x; i < m; i += kReduceThreads) {
-    double v = 0.0;
-    for (int s = 0; s < splits; ++s) v += part[(int64_t(s) * NV + OFF) * m + i];
-    acc += v;
-  }
+#pragma unroll 8
+  for (int64_t i = threadIdx.x; i < m; i += kReduceThreads) acc += v[i];
   red[threadIdx.x] = acc;
   __syncthreads();
   for (int w = kReduceThreads / 2; w > 0; w >>= 1) {
@@ -425,11 +451,18 @@ __global__ void write_scalar_kernel(double* out, double v) { out[0] = v; }
 
 template <class T, int KIND, int NV>
 int finalize_vec(const double* part, int splits, int64_t m, const Rec<T>* tgt, double* out,
-                 double* out2, cudaStream_t st, double* out3 = nullptr) {
+                 double* out2, cudaStream_t st, double* out3 = nullptr,
+                 double* scalar = nullptr) {
   if (m <= 0) return VPM_OK;
-  const int threads = 256;
-  finalize_vec_kernel<T, KIND, NV><<<unsigned((m + threads - 1) / threads), threads, 0, st>>>(
-      part, splits, m, tgt, out, out2, out3);
+  const SetsFinalize<T, KIND, NV> fin{tgt, out, out2, out3, scalar};
+  if (splits >= kSetLanesMinSplits && m <= kSetLanesMaxTargets) {
+    finalize_sets_kernel<NV, NV, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
+        part, SplitSets{splits}, m, fin);
+  } else {
+    const int threads = 256;
+    finalize_vec_kernel<T, KIND, NV>
+        <<<unsigned((m + threads - 1) / threads), threads, 0, st>>>(part, splits, m, fin);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "finalize launch");
   return VPM_OK;
@@ -563,6 +596,13 @@ struct RotSweep {
     return full * ((m * nt + slots - 1) / slots) + (rem * nt + slots - 1) / slots;
   }
 
+  // Creates the side stream now, outside any stream capture of the launch that follows.
+  static int prepare_side() {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    SideStream* ss = nullptr;
+    return side_stream(&ss);
+  }
+
   // eff_out: the fraction of whole waves the chosen launches fill (ideal waves / waves)
   static int plan(int64_t n, Plan* p, size_t max_partial_bytes, double* eff_out = nullptr) {
     DevInfo d;
@@ -618,10 +658,7 @@ struct RotSweep {
     // 1-2 % at 49152.  At large n that launch is a few tenths of a percent of the sweep.
     const bool beside = best_w <= 64 && sets(best_m, true) * set_bytes(n) <= max_partial_bytes;
     if (beside) {
-      // create the side stream now, outside any stream capture of the launch that follows
-      std::lock_guard<std::mutex> lk(g_side_mu);
-      SideStream* ss = nullptr;
-      rc = side_stream(&ss);
+      rc = prepare_side();
       if (rc) return rc;
     }
     p->diag_beside = beside ? 1 : 0;
@@ -836,15 +873,14 @@ __global__ void pack_grad_kernel(const double* __restrict__ pos, const double* _
   out[i] = r;
 }
 
+// The gradients of particle i from its summed values v.
 template <class E, int NV, bool PSE>
-__global__ void finalize_vjp_kernel(const double* __restrict__ part, int splits, int64_t m,
-                                    const RecG<E>* __restrict__ tgt, double* __restrict__ gx,
-                                    double* __restrict__ ga, double* __restrict__ gsig,
-                                    double* __restrict__ gnu) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  double v[NV];
-  sum_splits<NV>(part, splits, m, i, v);
+__device__ __forceinline__ void finalize_vjp_values(const double (&v)[NV],
+                                                    const RecG<E>* __restrict__ tgt, int64_t i,
+                                                    double* __restrict__ gx,
+                                                    double* __restrict__ ga,
+                                                    double* __restrict__ gsig,
+                                                    double* __restrict__ gnu) {
   const RecG<E>& t = tgt[i];
   const double ax = elem(t.ax), ay = elem(t.ay), az = elem(t.az);
   const double ux = elem(t.ux), uy = elem(t.uy), uz = elem(t.uz);
@@ -872,6 +908,38 @@ __global__ void finalize_vjp_kernel(const double* __restrict__ part, int splits,
   if (gnu) gnu[i] = PSE ? 105.0 * v[VJ_NU] : 0.0;
 }
 
+template <class E, bool PSE>
+struct SetsFinalizeVjp {
+  const RecG<E>* rec;
+  double *gx, *ga, *gs, *gnu;
+  static constexpr int NV = OpRhsVjp<E, false, PSE>::NV;
+  __device__ __forceinline__ void write(const double (&v)[NV], int64_t i) const {
+    finalize_vjp_values<E, NV, PSE>(v, rec, i, gx, ga, gs, gnu);
+  }
+};
+
+template <class E, bool PSE>
+__global__ void finalize_vjp_kernel(const double* __restrict__ part, int splits, int64_t m,
+                                    const SetsFinalizeVjp<E, PSE> fin) {
+  constexpr int NV = SetsFinalizeVjp<E, PSE>::NV;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  double v[NV];
+  sum_splits<NV>(part, splits, m, i, v);
+  fin.write(v, i);
+}
+
+template <class E, bool PSE>
+void finalize_vjp(const double* part, int splits, int64_t m, const SetsFinalizeVjp<E, PSE>& fin,
+                  cudaStream_t st) {
+  constexpr int NV = SetsFinalizeVjp<E, PSE>::NV;
+  if (splits >= kSetLanesMinSplits && m <= kSetLanesMaxTargets)
+    finalize_sets_kernel<NV, NV, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
+        part, SplitSets{splits}, m, fin);
+  else
+    finalize_vjp_kernel<E, PSE><<<unsigned((m + 255) / 256), 256, 0, st>>>(part, splits, m, fin);
+}
+
 __global__ void finalize_kegrad_kernel(const double* __restrict__ part, int splits, int64_t m,
                                        double* __restrict__ gx, double* __restrict__ ga,
                                        double* __restrict__ gsig) {
@@ -887,6 +955,98 @@ __global__ void finalize_kegrad_kernel(const double* __restrict__ part, int spli
   ga[3 * i + 1] = c * v[4];
   ga[3 * i + 2] = c * v[5];
   gsig[i] = 0.5 * c * v[6];
+}
+
+// ---- FP64 both-sides sweep in one launch (vpm_circle.cuh) ------------------------------------
+// Lower end of its range, a sixth of the both-sides threshold (so that vpm_set_symmetric_min_n
+// moves both): 4096 particles by default.  Measured against the one-sided sweeps (us, velocity /
+// fused / stretching / PSE / LES / adjoint): 36 / 58 / 43 / 31 / 73 / 90 against 26 / 39 / 35 / 27
+// / 73 / 80 at 3072, 37 / 61 / 44 / 32 / 92 / 115 against 39 / 64 / 59 / 39 / 106 / 149 at 4096,
+// 50 / 82 / 61 / 43 / 134 / 167 against 61 / 92 / 85 / 57 / 150 / 219 at 5000.
+int64_t circle_min_n() { return g_sym_min_n.load() / 6; }
+
+template <class Op>
+struct CircleSweep {
+  static constexpr int NV = Op::NV;
+  static constexpr int NJ = Op::kSymFrom;
+  static constexpr int kTile = rot_tile<Op>();
+  static constexpr size_t kSmem = lists64_smem_bytes<Op>();
+
+  static int prepare(int* occ) {
+    const void* fn = reinterpret_cast<const void*>(&rot64_lists_kernel<Op, CircleLists>);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    const auto key = std::make_pair(fn, dev);
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_occ.find(key);
+    if (it == g_occ.end()) {
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem));
+      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(circle sweep)");
+      int o = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kRotThreads, kSmem);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+      it = g_occ.emplace(key, o > 0 ? o : 1).first;
+    }
+    *occ = it->second;
+    return VPM_OK;
+  }
+
+  // Fills the plan; leaves p->circle 0 where the sets exceed the budget.
+  static int plan(int64_t n, Plan* p, size_t max_partial_bytes) {
+    DevInfo d;
+    int occ = 1;
+    int rc = device_info(&d);
+    if (!rc) rc = prepare(&occ);
+    if (rc) return rc;
+    const CircleLists l(n, kTile);
+    p->shares = Shares::make(l.total(), int64_t(d.sms) * occ);
+    const int64_t sets = target_sets(l, p->shares) + l.half;
+    if (size_t(sets) * NV * size_t(n) * sizeof(double) > max_partial_bytes) return VPM_OK;
+    p->circle = 1;
+    p->tblocks = l.nt;
+    p->splits = int(sets);
+    p->chunk = n;
+    p->smem = kSmem;
+    p->threads = kRotThreads;
+    p->r = 2 * Op::kP;
+    p->nv = NV;
+    return VPM_OK;
+  }
+
+  // acc: [p.splits][NV][n]; fin.write(v, i) takes the sums of particle i.
+  template <class Finalize>
+  static int launch(const Plan& p, const void* rec, int64_t n, double* acc, const Finalize& fin,
+                    cudaStream_t st) {
+    const CircleLists l(n, kTile);
+    const int tsets = p.splits - l.half;
+    const Sweep64Args a{rec, int(n), p.shares, acc, acc + int64_t(tsets) * NV * n};
+    rot64_lists_kernel<Op, CircleLists>
+        <<<unsigned(p.shares.blocks()), kRotThreads, kSmem, st>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "circle sweep launch");
+    const CircleSets sets{l, p.shares, kTile, tsets, n};
+    finalize_sets_kernel<NV, NJ, CircleSets, Finalize>
+        <<<unsigned((n + 31) / 32), 32 * kSetLanes, 0, st>>>(acc, sets, n, fin);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
+  }
+};
+
+
+// The FP64 plan of a self sum of n particles on the both-sides schedules, if it takes one
+// (p->circle or p->pairs set).  MULTI: from the threshold on the sum takes the many-launch sweep;
+// otherwise the circle at all sizes its sets fit.
+template <class Op, bool MULTI>
+int plan_both64(int64_t m, int64_t n, Plan* p, size_t mpb) {
+  if (m != n) return VPM_OK;
+  const bool large = RotSweep<Op>::usable(m, n, mpb);
+  if (n > 0 && n >= circle_min_n() && n < (int64_t(1) << 30) && RotSweep<Op>::tiles(n) >= 2 &&
+      !(MULTI && n >= g_sym_min_n.load())) {
+    int rc = CircleSweep<Op>::plan(n, p, mpb);
+    if (rc || p->circle) return rc;
+  }
+  return large ? RotSweep<Op>::plan(n, p, mpb) : VPM_OK;
 }
 
 // ---- small sums in one launch (vpm_small.cuh) ---------------------------------------------
@@ -1011,6 +1171,9 @@ struct Ops {
   using VelBoth64 = OpVelBoth64<UC>;                // FP64 only
   using PseBoth64 = OpPseBoth64<UC>;                // FP64 only
   using LesStepBoth64 = OpLesStepBoth64<UC>;        // FP64 only
+  using StretchBoth64 = OpStretchBoth64<UC>;        // FP64 only
+  using RhsVjpBoth64 = OpRhsVjpBoth64<false>;       // FP64 only
+  using RhsVjpPseBoth64 = OpRhsVjpBoth64<true>;     // FP64 only
   using VelBoth = OpVelBoth<REFINE, UC>;                // FP32 only
   using PseBoth = OpPseBoth<REFINE, UC>;                // FP32 only
   using LesStepBoth = OpLesStepBoth<REFINE, UC>;        // FP32 only
@@ -1032,40 +1195,44 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
         if (RotSweep<typename O::VelBoth>::usable(m, n, mpb))
           return RotSweep<typename O::VelBoth>::plan(n, p, mpb);
       } else {
-        if (RotSweep<typename O::VelBoth64>::usable(m, n, mpb))
-          return RotSweep<typename O::VelBoth64>::plan(n, p, mpb);
+        const int rc = plan_both64<typename O::VelBoth64, true>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::Vel, T, FIN_VEL>(m, n, p, mpb);
     case VPM_OP_TOTAL_HELICITY:
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarHel>::plan(n, p);
       }
-      return Sweep<typename O::Vel, T>::plan(m, n, p, mpb);
+      return Sweep<typename O::Vel, T>::plan(m, n, p, mpb, kMinChunkScalar);
     case VPM_OP_INDUCED_VELOCITY_AT:
       return plan_vector<typename O::VelAt, T, FIN_VEL>(m, n, p, mpb);
     case VPM_OP_VORTICITY_FIELD_AT:
       return plan_vector<typename O::VortAt, T, FIN_VORT>(m, n, p, mpb);
     case VPM_OP_STRENGTH_GRADIENTS:
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        const int rc = plan_both64<typename O::StretchBoth64, false>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
+      }
       return plan_vector<typename O::Stretch, T, FIN_STRETCH>(m, n, p, mpb);
     case VPM_OP_STRENGTH_GRADIENTS_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::PseBoth>::usable(m, n, mpb))
           return RotSweep<typename O::PseBoth>::plan(n, p, mpb);
       } else {
-        if (RotSweep<typename O::PseBoth64>::usable(m, n, mpb))
-          return RotSweep<typename O::PseBoth64>::plan(n, p, mpb);
+        const int rc = plan_both64<typename O::PseBoth64, true>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::Pse, T, FIN_PSE>(m, n, p, mpb);
     case VPM_OP_TOTAL_KINETIC_ENERGY:
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarKe>::plan(n, p);
       }
-      return Sweep<typename O::Ke, T>::plan(m, n, p, mpb);
+      return Sweep<typename O::Ke, T>::plan(m, n, p, mpb, kMinChunkScalar);
     case VPM_OP_TOTAL_ENSTROPHY:
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarEns>::plan(n, p);
       }
-      return Sweep<typename O::Ens, T>::plan(m, n, p, mpb);
+      return Sweep<typename O::Ens, T>::plan(m, n, p, mpb, kMinChunkScalar);
     case VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::VelStretchBoth>::usable(m, n, mpb)) {
@@ -1101,8 +1268,8 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
           return VPM_OK;
         }
       } else {
-        if (RotSweep<typename O::VelStretchBoth64>::usable(m, n, mpb))
-          return RotSweep<typename O::VelStretchBoth64>::plan(n, p, mpb);
+        const int rc = plan_both64<typename O::VelStretchBoth64, true>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::VelStretch, T, FIN_VELSTRETCH>(m, n, p, mpb);
     case VPM_OP_LES_STEP_SUMS:
@@ -1110,20 +1277,26 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
         if (RotSweep<typename O::LesStepBoth>::usable(m, n, mpb))
           return RotSweep<typename O::LesStepBoth>::plan(n, p, mpb);
       } else {
-        if (RotSweep<typename O::LesStepBoth64>::usable(m, n, mpb))
-          return RotSweep<typename O::LesStepBoth64>::plan(n, p, mpb);
+        const int rc = plan_both64<typename O::LesStepBoth64, true>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
       }
       return Sweep<typename O::LesStep, T>::plan(m, n, p, mpb);
     case VPM_OP_RHS_VJP:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::RhsVjpBoth>::usable(m, n, mpb))
           return RotSweep<typename O::RhsVjpBoth>::plan(n, p, mpb);
+      } else {
+        const int rc = plan_both64<typename O::RhsVjpBoth64, false>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
       }
       return Sweep<typename O::RhsVjp, T>::plan(m, n, p, mpb);
     case VPM_OP_RHS_VJP_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::RhsVjpPseBoth>::usable(m, n, mpb))
           return RotSweep<typename O::RhsVjpPseBoth>::plan(n, p, mpb);
+      } else {
+        const int rc = plan_both64<typename O::RhsVjpPseBoth64, false>(m, n, p, mpb);
+        if (rc || p->circle || p->pairs) return rc;
       }
       return Sweep<typename O::RhsVjpPse, T>::plan(m, n, p, mpb);
     case VPM_OP_KINETIC_ENERGY_GRAD:
@@ -1137,6 +1310,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
 
 struct Layout {
   size_t src_off = 0, tgt_off = 0, part_off = 0, total = 0;
+  size_t scalar_off = 0;  // LES step sums: one scalar per target, reduced after the finalize
 };
 
 template <class T>
@@ -1155,6 +1329,8 @@ Layout layout_for(int op, const Plan& p, int64_t m, int64_t n) {
   if (is_probe(op)) off = align_up(off + size_t(m > 0 ? m : 0) * sizeof(Rec<T>));
   L.part_off = off;
   off = align_up(off + size_t(p.splits) * p.nv * size_t(m > 0 ? m : 0) * sizeof(double));
+  L.scalar_off = off;
+  if (op == VPM_OP_LES_STEP_SUMS) off = align_up(off + size_t(m > 0 ? m : 0) * sizeof(double));
   L.total = off;
   return L;
 }
@@ -1262,6 +1438,12 @@ int run(const Call& c) {
   switch (c.op) {
     case VPM_OP_SELFINDUCED_VELOCITY:
       rc = VPM_OK;
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (p.circle)
+          return CircleSweep<typename O::VelBoth64>::launch(
+              p, src, c.n, part, SetsFinalize<double, FIN_VEL, 3>{src, c.out, nullptr, nullptr, nullptr},
+              c.st);
+      }
       if (p.pairs) {  // m == n: the targets are all the records (tgt_begin == 0)
         if constexpr (LaneTraits<T>::kLanes == 2)
           rc = RotSweep<typename O::VelBoth>::launch(p, src, c.n, part, c.st);
@@ -1281,12 +1463,27 @@ int run(const Call& c) {
       if (!rc) rc = finalize_vec<T, FIN_VORT, 3>(part, p.splits, c.m, tgt, c.out, nullptr, c.st);
       return rc;
     case VPM_OP_STRENGTH_GRADIENTS:
-      rc = Sweep<typename O::Stretch, T>::launch(p, tgt, c.m, c.tgt_begin, src, c.n, part, c.st);
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (p.circle)
+          return CircleSweep<typename O::StretchBoth64>::launch(
+              p, src, c.n, part,
+              SetsFinalize<double, FIN_STRETCH, 6>{src, c.out, nullptr, nullptr, nullptr}, c.st);
+        if (p.pairs) rc = RotSweep<typename O::StretchBoth64>::launch(p, src, c.n, part, c.st);
+      }
+      if (!p.pairs)
+        rc = Sweep<typename O::Stretch, T>::launch(p, tgt, c.m, c.tgt_begin, src, c.n, part,
+                                                   c.st);
       if (!rc)
         rc = finalize_vec<T, FIN_STRETCH, 6>(part, p.splits, c.m, tgt, c.out, nullptr, c.st);
       return rc;
     case VPM_OP_STRENGTH_GRADIENTS_PSE:
       rc = VPM_OK;
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (p.circle)
+          return CircleSweep<typename O::PseBoth64>::launch(
+              p, src, c.n, part, SetsFinalize<double, FIN_PSE, 3>{src, c.out, nullptr, nullptr, nullptr},
+              c.st);
+      }
       if (p.pairs) {
         if constexpr (LaneTraits<T>::kLanes == 2)
           rc = RotSweep<typename O::PseBoth>::launch(p, src, c.n, part, c.st);
@@ -1308,6 +1505,10 @@ int run(const Call& c) {
         else
           rc = Sweep<typename O::VelStretch, T>::launch(p, tgt, c.m, c.tgt_begin, src, c.n,
                                                         part, c.st);
+      } else if (p.circle) {
+        return CircleSweep<typename O::VelStretchBoth64>::launch(
+            p, src, c.n, part,
+            SetsFinalize<double, FIN_VELSTRETCH, 9>{src, c.out, c.out2, nullptr, nullptr}, c.st);
       } else if (p.pairs) {
         rc = RotSweep<typename O::VelStretchBoth64>::launch(p, src, c.n, part, c.st);
       } else {
@@ -1326,28 +1527,37 @@ int run(const Call& c) {
           rc = RotSweep<typename O::LesStepBoth>::launch(p, src, c.n, part, c.st);
         else
           rc = RotSweep<typename O::LesStepBoth64>::launch(p, src, c.n, part, c.st);
+        if (rc) return rc;
       }
-      if (!p.pairs) rc = Sweep<Op, T>::launch(p, tgt, c.m, c.tgt_begin, src, c.n, part, c.st);
-      if (rc) return rc;
       double scale = 1.0 / (8.0 * kPi);
       if (c.ref_extra_4pi) scale /= 4.0 * kPi;
-      if (p.pairs) {
-        // both sides: the per-target scalar sum_j ke (a_i . a_j) (value 12), taken once per
-        // unordered pair, so the sum is doubled
-        constexpr int NVB = O::LesStepBoth::NV;
-        static_assert(O::LesStepBoth64::NV == NVB, "one row layout for both precisions");
-        rc = finalize_vec<T, FIN_LES, NVB>(part, p.splits, c.m, tgt, c.out, c.out2, c.st,
-                                           c.out3);
-        if (rc) return rc;
-        finalize_sum_kernel<NVB, 12><<<1, kReduceThreads, 0, c.st>>>(part, p.splits, c.m,
-                                                                     2.0 * scale, c.out4);
-      } else {
-        rc = finalize_vec<T, FIN_LES, Op::NV>(part, p.splits, c.m, tgt, c.out, c.out2, c.st,
-                                               c.out3);
-        if (rc) return rc;
-        finalize_dot_kernel<T, Op::NV, 12><<<1, kReduceThreads, 0, c.st>>>(part, p.splits, c.m,
-                                                                            tgt, scale, c.out4);
+      // every target's scalar a_i . E_i: from the both-sides sums sum_j ke (a_i . a_j) (value
+      // 12), taken once per unordered pair, so doubled
+      double* scalar = reinterpret_cast<double*>(ws + L.scalar_off);
+      constexpr int NVB = O::LesStepBoth::NV;
+      static_assert(O::LesStepBoth64::NV == NVB, "one row layout for both precisions");
+      bool done = false;
+      if constexpr (LaneTraits<T>::kLanes == 1) {
+        if (p.circle) {
+          rc = CircleSweep<typename O::LesStepBoth64>::launch(
+              p, src, c.n, part,
+              SetsFinalize<double, FIN_LES, NVB>{src, c.out, c.out2, c.out3, scalar}, c.st);
+          scale *= 2.0;
+          done = true;
+        }
       }
+      if (!done && p.pairs) {
+        rc = finalize_vec<T, FIN_LES, NVB>(part, p.splits, c.m, tgt, c.out, c.out2, c.st, c.out3,
+                                           scalar);
+        scale *= 2.0;
+      } else if (!done) {
+        rc = Sweep<Op, T>::launch(p, tgt, c.m, c.tgt_begin, src, c.n, part, c.st);
+        if (!rc)
+          rc = finalize_vec<T, FIN_LES, Op::NV>(part, p.splits, c.m, tgt, c.out, c.out2, c.st,
+                                                c.out3, scalar);
+      }
+      if (rc) return rc;
+      finalize_sum_kernel<<<1, kReduceThreads, 0, c.st>>>(scalar, c.m, scale, c.out4);
       cudaError_t e = cudaGetLastError();
       return e == cudaSuccess ? VPM_OK : cuda_fail(e, "reduce launch");
     }
@@ -1556,21 +1766,31 @@ int run_grad(const GradCall& c) {
     rc = VPM_OK;
     if constexpr (LaneTraits<T>::kLanes == 2) {
       if (p.pairs) rc = RotSweep<typename O::RhsVjpPseBoth>::launch(p, rec, c.n, part, c.st);
+    } else {
+      if (p.circle)
+        return CircleSweep<typename O::RhsVjpPseBoth64>::launch(
+            p, rec, c.n, part, SetsFinalizeVjp<double, true>{rec, c.ox, c.oa, c.os, c.onu}, c.st);
+      if (p.pairs) rc = RotSweep<typename O::RhsVjpPseBoth64>::launch(p, rec, c.n, part, c.st);
     }
     if (!p.pairs)
       rc = Sweep<typename O::RhsVjpPse, T>::launch(p, rec, c.n, 0, rec, c.n, part, c.st);
     if (rc) return rc;
-    finalize_vjp_kernel<T, O::RhsVjpPse::NV, true>
-        <<<blocks, 256, 0, c.st>>>(part, p.splits, c.n, rec, c.ox, c.oa, c.os, c.onu);
+    finalize_vjp<T, true>(part, p.splits, c.n, SetsFinalizeVjp<T, true>{rec, c.ox, c.oa, c.os, c.onu},
+                        c.st);
   } else {
     rc = VPM_OK;
     if constexpr (LaneTraits<T>::kLanes == 2) {
       if (p.pairs) rc = RotSweep<typename O::RhsVjpBoth>::launch(p, rec, c.n, part, c.st);
+    } else {
+      if (p.circle)
+        return CircleSweep<typename O::RhsVjpBoth64>::launch(
+            p, rec, c.n, part, SetsFinalizeVjp<double, false>{rec, c.ox, c.oa, c.os, c.onu}, c.st);
+      if (p.pairs) rc = RotSweep<typename O::RhsVjpBoth64>::launch(p, rec, c.n, part, c.st);
     }
     if (!p.pairs) rc = Sweep<typename O::RhsVjp, T>::launch(p, rec, c.n, 0, rec, c.n, part, c.st);
     if (rc) return rc;
-    finalize_vjp_kernel<T, O::RhsVjp::NV, false>
-        <<<blocks, 256, 0, c.st>>>(part, p.splits, c.n, rec, c.ox, c.oa, c.os, c.onu);
+    finalize_vjp<T, false>(part, p.splits, c.n, SetsFinalizeVjp<T, false>{rec, c.ox, c.oa, c.os, c.onu},
+                        c.st);
   }
   e = cudaGetLastError();
   return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
@@ -2043,6 +2263,7 @@ int64_t vpm_sweep_launches(int op, int precision, int64_t m, int64_t n) {
     const int64_t npairs = p.tblocks / 2;
     return 3 + (npairs + p.pairs - 1) / p.pairs;
   }
+  if (p.circle) return op == VPM_OP_LES_STEP_SUMS ? 3 : 2;
   if (p.small) return 1;  // pack, sweep and finalize in one
   return 2;  // sweep, finalize (or the single-block reduction of a scalar)
 }

@@ -354,6 +354,47 @@ struct OpVelBoth : RotStd<OpVel<float2, REFINE, UC>, UC> {
   }
 };
 
+// Stretching alone, both sides of the pair (FP64 only): the fused sum's A and B.
+template <bool UC>
+struct OpStretchBoth {
+  static constexpr int NV = 6;
+  static constexpr int kSymFrom = NV;
+  static constexpr bool kCustomDiag = false;
+  template <class W>
+  __device__ __forceinline__ static void pair2(const Tgt<W>& t, W* acc, W* jv,
+                                               const Src<W>& s) {
+    using V = W;
+    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
+    V sg, s2;
+    pair_core<UC>(t, s, sg, s2);
+    const V x = fma(rx, rx, fma(ry, ry, fma(rz, rz, s2)));
+    const V y = rsqrt_lane<false>(x);
+    const V y2 = y * y;
+    const V y5 = (y2 * y2) * y;
+    const V t1 = fma(splat<V>(1.5), s2, x);
+    const V g = t1 * y5;
+    const V f = (t1 + s2) * (y5 * y2);
+    const V dx = s.ax - t.ax, dy = s.ay - t.ay, dz = s.az - t.az;
+    acc[0] = fma(g, dx, acc[0]);
+    acc[1] = fma(g, dy, acc[1]);
+    acc[2] = fma(g, dz, acc[2]);
+    const V wx = fma(dy, t.az, -(dz * t.ay));  // d x a_i
+    const V wy = fma(dz, t.ax, -(dx * t.az));
+    const V wz = fma(dx, t.ay, -(dy * t.ax));
+    const V h = f * fma(rx, wx, fma(ry, wy, rz * wz));
+    acc[3] = fma(h, rx, acc[3]);
+    acc[4] = fma(h, ry, acc[4]);
+    acc[5] = fma(h, rz, acc[5]);
+    // source side, accumulated with the opposite sign (negated when it is stored)
+    jv[0] = fma(g, dx, jv[0]);
+    jv[1] = fma(g, dy, jv[1]);
+    jv[2] = fma(g, dz, jv[2]);
+    jv[3] = fma(h, rx, jv[3]);
+    jv[4] = fma(h, ry, jv[4]);
+    jv[5] = fma(h, rz, jv[5]);
+  }
+};
+
 // PSE diffusion, both sides of the pair (FP32x2 lanes): the kernel value k is symmetric and
 // the exchange antisymmetric, P_j += -k (a_j - a_i); nu of each particle is applied by the
 // finalize.
@@ -538,14 +579,17 @@ struct OpLesStepBoth : RotStd<OpLesStep<float2, REFINE, UC>, UC> {
 // symmetric too, and particle l takes dL/dnu'_l += k s'_l.(a_k - a_l), sum k and
 // sum k nu'_k s'_k; the lane carries nu' as a 17th value.  The 18 sums fit two targets per
 // lane (VPM_ROTGP_P).
+template <class V>
+struct TgtGM : TgtG<V> {
+  V mx, my, mz;  // m_k = a_k x s'_k
+};
+
 template <bool REFINE, bool PSE>
 struct OpRhsVjpBoth {
   using V = float2;
   using Record = RecG<float2>;
   using OneSided = OpRhsVjp<float2, REFINE, PSE>;
-  struct TgtT : TgtG<float2> {
-    float2 mx, my, mz;  // m_k = a_k x s'_k
-  };
+  using TgtT = TgtGM<float2>;
   using SrcT = SrcG<float2>;
   struct Lane {
     float x, y, z, s, ax, ay, az, ux, uy, uz, gx, gy, gz, mx, my, mz, nu;  // nu: 105 nu
@@ -605,7 +649,11 @@ struct OpRhsVjpBoth {
   }
   __device__ __forceinline__ static constexpr bool carried(int v) { return PSE || v != VJ_NU; }
 
-  __device__ __forceinline__ static void pair2(const TgtT& t, V* acc, V* jv, const SrcT& s) {
+  // in any lane type (float2 here; double in the FP64 operator below)
+  template <class W>
+  __device__ __forceinline__ static void pair2(const TgtGM<W>& t, W* acc, W* jv,
+                                               const SrcG<W>& s) {
+    using V = W;
     const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
     const V sg = fma(s.s, splat<V>(0.5), t.hs);
     const V s2 = sg * sg;
@@ -942,11 +990,15 @@ rot_sweep_kernel(const RotArgs a) {
 #ifndef VPM_ROT64_MINB
 #define VPM_ROT64_MINB 2
 #endif
+// Tuning of the FP64 builds, Gpairs/s at 131072 particles (fused / velocity / PSE): R = 4, two
+// CTAs per SM and four steps unrolled 459 / 766 / 967; two steps unrolled and (velocity, PSE)
+// three CTAs per SM 456 / 742 / 945; R = 2 and three CTAs 427 / 695 / 842; R = 2 and four CTAs
+// 410 / 675 / 827; R = 6 426 (one CTA) / 765 / 927.  Two warps per scheduler with four targets'
+// chains each hide more of the FP64 latency than more warps with fewer, whose shuffles double.
 
 // Both32: the FP32 both-sides operator whose pair2 (a template in the lane type) gives the
 // pair terms; OneSided64: the one-sided FP64 operator of the diagonal tiles.
-template <class Both32, class OneSided64, bool UC, int MINB = VPM_ROT64_MINB,
-          int P = VPM_ROT64_P>
+template <class Both32, class OneSided64, bool UC, int UNROLL = 4, int P = VPM_ROT64_P>
 struct OpBoth64 {
   using V = double;
   using Record = Rec<double>;
@@ -956,10 +1008,14 @@ struct OpBoth64 {
   static constexpr bool kFP64 = true;
   static constexpr int NV = Both32::NV;
   static constexpr int kP = P;  // rot_tile: 64 kP warps = 32 R warps
-  static constexpr int kMinBlocks = MINB;
+  static constexpr int kMinBlocks = VPM_ROT64_MINB;
+  static constexpr int kUnroll = UNROLL;  // of a batch's 32 steps
+  static constexpr bool kPrefetch = true;  // the next batch's source loads under this one's sums
   // values from kSymFrom on are taken once per unordered pair on the target side only
   static constexpr int kSymFrom = Both32::kSymFrom;
   static constexpr bool kUniformCore = UC;
+  // every source-side sum is carried and stored
+  __device__ __forceinline__ static constexpr bool carried(int) { return true; }
   __device__ __forceinline__ static SrcT load(const Record* rec, int64_t j, int64_t n) {
     if (j < n) return load_src<double>(rec[j]);
     // far and without strength: r^2 = 1e220 stays finite and y^3 = 1e-330 underflows to 0,
@@ -975,6 +1031,14 @@ struct OpBoth64 {
     c.ay = __shfl_sync(0xffffffffu, c.ay, src_lane);
     c.az = __shfl_sync(0xffffffffu, c.az, src_lane);
   }
+  // target i (i < n), or one past n like a source past n
+  __device__ __forceinline__ static TgtT target(const Record* rec, int64_t i, int64_t n) {
+    if (i < n) {
+      const Record* rp = rec + i;
+      return make_tgt(&rp);
+    }
+    return TgtT{1e110, 1e110, 1e110, 0.5, 0.0, 0.0, 0.0, 1.0, 1.0, 1.0};
+  }
   __device__ __forceinline__ static void uniform_core(TgtT& t, const Record* rec) {
     const double sc = rec[0].s, s2 = sc * sc;
     t.sc = sc;
@@ -985,7 +1049,8 @@ struct OpBoth64 {
                                                const SrcT& s) {
     Both32::pair2(t, acc, jv, s);
   }
-  __device__ __forceinline__ static void diag(const TgtT& t, double* acc, const SrcT& s) {
+  __device__ __forceinline__ static void diag(const TgtT& t, double* acc, const SrcT& s,
+                                              const int64_t*, int64_t) {
     if constexpr (Both32::kCustomDiag)
       Both32::diag(t, acc, s, nullptr, 0);
     else
@@ -995,15 +1060,74 @@ struct OpBoth64 {
 template <bool UC>
 using OpVelStretchBoth64 =
     OpBoth64<OpVelStretchBoth<false, UC>, OpVelStretch<double, false, UC>, UC>;
-// the three-sum operators fit three CTAs per SM
 template <bool UC>
-using OpVelBoth64 = OpBoth64<OpVelBoth<false, UC>, OpVel<double, false, UC>, UC, 3>;
+using OpVelBoth64 = OpBoth64<OpVelBoth<false, UC>, OpVel<double, false, UC>, UC>;
 template <bool UC>
-using OpPseBoth64 = OpBoth64<OpPseBoth<false, UC>, OpPse<double, false, UC>, UC, 3>;
+using OpPseBoth64 = OpBoth64<OpPseBoth<false, UC>, OpPse<double, false, UC>, UC>;
 // the LES step's 13 sums: two FP64 targets per lane (256-particle tiles)
 template <bool UC>
 using OpLesStepBoth64 =
     OpBoth64<OpLesStepBoth<false, UC>, OpLesStep<double, false, UC>, UC, 2, 1>;
+template <bool UC>
+using OpStretchBoth64 = OpBoth64<OpStretchBoth<UC>, OpStretch<double, false, UC>, UC>;
+
+// The adjoint of (u, S [+ P]) in FP64 (OpRhsVjpBoth's pair terms): 14 or 18 sums and 16 or 17
+// travelling values leave room for two targets per lane.
+template <bool PSE>
+struct OpRhsVjpBoth64 {
+  using V = double;
+  using Record = RecG<double>;
+  using Both32 = OpRhsVjpBoth<false, PSE>;
+  using OneSided = OpRhsVjp<double, false, PSE>;
+  using TgtT = TgtGM<double>;
+  using SrcT = SrcG<double>;
+  static constexpr bool kFP64 = true;
+  static constexpr int NV = OneSided::NV;
+  static constexpr int kP = 1;
+  static constexpr int kMinBlocks = 2;
+  static constexpr int kUnroll = 1;
+  static constexpr bool kPrefetch = false;  // 17 values of registers: loaded at the batch's start
+  static constexpr int kSymFrom = NV;
+  static constexpr bool kUniformCore = false;
+  __device__ __forceinline__ static constexpr bool carried(int v) { return PSE || v != VJ_NU; }
+  __device__ __forceinline__ static void uniform_core(TgtT&, const Record*) {}
+  __device__ __forceinline__ static SrcT load(const Record* rec, int64_t j, int64_t n) {
+    if (j < n) return load_srcg(rec[j]);
+    SrcT s{};  // far and without strength or cotangents (see OpBoth64::load)
+    s.x = s.y = s.z = 1e110;
+    s.s = 1.0;
+    return s;
+  }
+  __device__ __forceinline__ static TgtT target(const Record* rec, int64_t i, int64_t n) {
+    TgtT t{};
+    if (i < n) {
+      const Record* rp = rec + i;
+      static_cast<TgtG<double>&>(t) = make_tgtg(&rp);
+      t.mx = rp->mx;
+      t.my = rp->my;
+      t.mz = rp->mz;
+    } else {
+      t.x = t.y = t.z = 1e110;
+      t.hs = 0.5;
+    }
+    return t;
+  }
+  __device__ __forceinline__ static void shuffle(SrcT& c, int src_lane) {
+    double* v[] = {&c.x,  &c.y,  &c.z,  &c.s,  &c.ax, &c.ay, &c.az, &c.ux, &c.uy,
+                   &c.uz, &c.gx, &c.gy, &c.gz, &c.mx, &c.my, &c.mz, &c.nu};
+#pragma unroll
+    for (int q = 0; q < Both32::kLaneValues; ++q)
+      *v[q] = __shfl_sync(0xffffffffu, *v[q], src_lane);
+  }
+  __device__ __forceinline__ static void pair2(const TgtT& t, double* acc, double* jv,
+                                               const SrcT& s) {
+    Both32::pair2(t, acc, jv, s);
+  }
+  __device__ __forceinline__ static void diag(const TgtT& t, double* acc, const SrcT& s,
+                                              const int64_t* ti, int64_t j) {
+    OneSided::pair(t, acc, s, ti, j);
+  }
+};
 
 template <class Op, bool DIAG>
 __global__ void __launch_bounds__(kRotThreads, Op::kMinBlocks)
@@ -1034,8 +1158,7 @@ rot64_sweep_kernel(const RotArgs a) {
   for (int r = 0; r < R; ++r) {
     ti[r] = i0 + warp * 32 * R + r * 32 + lane;
     // past n only in the (one-sided) diagonal tiles, as in rot_sweep_kernel
-    const Record* rp = rec + (ti[r] < a.n ? ti[r] : a.n - 1);
-    tg[r] = make_tgt(&rp);
+    tg[r] = Op::target(rec, ti[r], a.n);
     if constexpr (Op::kUniformCore) Op::uniform_core(tg[r], rec);
   }
   double acc[R][NV];
@@ -1046,19 +1169,21 @@ rot64_sweep_kernel(const RotArgs a) {
 
   const int nb = (cnt + 31) / 32;
   const int src_lane = (lane + 1) & 31;
-  typename Op::SrcT nxt = Op::load(rec, j0 + lane, j0 + cnt);
+  typename Op::SrcT nxt;
+  if (Op::kPrefetch) nxt = Op::load(rec, j0 + lane, j0 + cnt);
   for (int b = 0; b < nb; ++b) {
-    typename Op::SrcT cur = nxt;  // the source this lane holds at step 0
-    if (b + 1 < nb) nxt = Op::load(rec, j0 + (b + 1) * 32 + lane, j0 + cnt);
+    // the source this lane holds at step 0
+    typename Op::SrcT cur = Op::kPrefetch ? nxt : Op::load(rec, j0 + b * 32 + lane, j0 + cnt);
+    if (Op::kPrefetch && b + 1 < nb) nxt = Op::load(rec, j0 + (b + 1) * 32 + lane, j0 + cnt);
     double jv[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) jv[v] = 0.0;
-#pragma unroll 2
+#pragma unroll Op::kUnroll
     for (int st = 0; st < 32; ++st) {
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if constexpr (DIAG)
-          Op::diag(tg[r], acc[r], cur);
+          Op::diag(tg[r], acc[r], cur, &ti[r], j0 + b * 32 + ((lane + st) & 31));
         else
           Op::pair2(tg[r], acc[r], jv, cur);
       }
@@ -1066,7 +1191,8 @@ rot64_sweep_kernel(const RotArgs a) {
       Op::shuffle(cur, src_lane);
       if constexpr (!DIAG) {
 #pragma unroll
-        for (int v = 0; v < NJ; ++v) jv[v] = __shfl_sync(0xffffffffu, jv[v], src_lane);
+        for (int v = 0; v < NJ; ++v)
+          if (Op::carried(v)) jv[v] = __shfl_sync(0xffffffffu, jv[v], src_lane);
       }
     }
     if constexpr (!DIAG) {
@@ -1077,7 +1203,7 @@ rot64_sweep_kernel(const RotArgs a) {
       const int nsrc = (cnt - b * 32 < 32) ? cnt - b * 32 : 32;
       for (int q = tid; q < 32 * NJ; q += kRotThreads) {
         const int v = q >> 5, jj = q & 31;
-        if (jj >= nsrc) continue;
+        if (jj >= nsrc || !Op::carried(v)) continue;
         double sum = 0.0;
 #pragma unroll
         for (int w = 0; w < kRotWarps; ++w) sum += jbuf[v * WT + w * 32 + jj];
