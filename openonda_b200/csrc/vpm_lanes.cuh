@@ -121,6 +121,16 @@ __device__ __forceinline__ float2 fma_if_gt(float2 a, double thr, float2 v, floa
   const float2 r = fma(v, w, acc);
   return make_float2(a.x > t ? r.x : acc.x, a.y > t ? r.y : acc.y);
 }
+// Whether every lane is surely above thr (false for NaN, and in FP64 for values that share thr's
+// high word or are infinite: those pairs take the exact test of fma_if_gt).
+__device__ __forceinline__ bool surely_gt(float2 a, double thr) {
+  const float t = float(thr);
+  return (a.x > t) & (a.y > t);
+}
+__device__ __forceinline__ bool surely_gt(double a, double thr) {
+  const unsigned above = unsigned(__double2hiint(thr)) + 1u;
+  return unsigned(__double2hiint(a)) - above < 0x7ff00000u - above;
+}
 // v except in the lanes whose target index equals j
 __device__ __forceinline__ double zero_if_self(double v, const int64_t* i, int64_t j) {
   return i[0] == j ? 0.0 : v;

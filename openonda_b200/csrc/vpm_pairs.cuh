@@ -110,9 +110,17 @@ __device__ __forceinline__ void pair_core(const Tgt<V>& t, const Src<V>& s, V& s
   }
 }
 
+// Targets per thread of the FP64 probe and filter sums (their FP32 forms: the default).  With the
+// branch-free root two targets' chains interleave: 466 -> 498 (velocity), 579 -> 600 (vorticity)
+// and 517 -> 537 Gpairs/s (test filter) at 65536 targets and sources against one per thread; the
+// self sums, which are one-sided only at small n, gain less and lose blocks.
+template <class V>
+constexpr int kProbeR = LaneTraits<V>::kLanes == 1 ? 2 : 0;
+
 // Record/lane plumbing shared by the operators on the standard 64-byte record.
 template <class V>
 struct PairOpBase {
+  static constexpr bool kGuarded = false;  // pairs within r^2 <= kRefEps are skipped (see OpVelAt)
   static constexpr int kR = 0;  // targets per thread: 0 = the precision's default
   // FP32 sources per FP64 carry fold of the one-sided sweep: 0 = the sweep's default (32)
   static constexpr int kWindow = 0;
@@ -147,44 +155,87 @@ struct OpVel : PairOpBase<V> {
 };
 
 // ---- probe velocity: source core sigma_j, pairs with r^2 <= 1e-8 skipped ----------------
+// Guarded operators split a pair into its term and its addition, so that the sweep can form the
+// terms of a few sources first and then test once that none of their pairs is to be skipped
+// (sweep_kernel): a compare per pair in place of a compare and three selects, and the sums stay
+// the same bits.  At 65536 targets and sources, Gpairs/s with selects / tests of 2 / 4 sources:
+// FP32c velocity 1117 / 1339 / 1341, vorticity 1447 / 1825 / 1776, test filter 1153 / 1538 /
+// 1572; FP64 498 / 555 / 576, 600 / 679 / 711, 537 / 635 / 646.
 template <class V, bool REFINE>
 struct OpVelAt : PairOpBase<V> {
+  static constexpr int kR = kProbeR<V>;
   static constexpr int NV = 3;
-  __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
-                                              const int64_t*, int64_t) {
+  static constexpr bool kGuarded = true;
+  static constexpr int kGuardGroup = 4;  // sources per test
+  struct Term {
+    V r2, g, cx, cy, cz;
+  };
+  __device__ __forceinline__ static Term term(const Tgt<V>& t, const Src<V>& s) {
     const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
     const V r2 = fma(rx, rx, fma(ry, ry, rz * rz));
     const V s2 = s.s * s.s;
     const V y = rsqrt_lane<REFINE>(r2 + s2);
     const V y2 = y * y;
     const V y5 = (y2 * y2) * y;
-    const V g = fma(splat<V>(2.5), s2, r2) * y5;
-    const V cx = fma(ry, s.az, -(rz * s.ay));
-    const V cy = fma(rz, s.ax, -(rx * s.az));
-    const V cz = fma(rx, s.ay, -(ry * s.ax));
-    acc[0] = fma_if_gt(r2, kRefEps, g, cx, acc[0]);
-    acc[1] = fma_if_gt(r2, kRefEps, g, cy, acc[1]);
-    acc[2] = fma_if_gt(r2, kRefEps, g, cz, acc[2]);
+    return Term{r2, fma(splat<V>(2.5), s2, r2) * y5, fma(ry, s.az, -(rz * s.ay)),
+                fma(rz, s.ax, -(rx * s.az)), fma(rx, s.ay, -(ry * s.ax))};
+  }
+  __device__ __forceinline__ static void add(V* acc, const Term& q, const Src<V>&) {
+    acc[0] = fma(q.g, q.cx, acc[0]);
+    acc[1] = fma(q.g, q.cy, acc[1]);
+    acc[2] = fma(q.g, q.cz, acc[2]);
+  }
+  __device__ __forceinline__ static void add_guarded(V* acc, const Term& q, const Src<V>&) {
+    acc[0] = fma_if_gt(q.r2, kRefEps, q.g, q.cx, acc[0]);
+    acc[1] = fma_if_gt(q.r2, kRefEps, q.g, q.cy, acc[1]);
+    acc[2] = fma_if_gt(q.r2, kRefEps, q.g, q.cz, acc[2]);
+  }
+  __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
+                                              const int64_t*, int64_t) {
+    add_guarded(acc, term(t, s), s);
   }
 };
+
+// The zeta kernel of the source core, s_j^4 (r^2 + s_j^2)^(-7/2).
+template <class V>
+struct ZetaTerm {
+  V r2, k;
+};
+template <class V, bool REFINE>
+__device__ __forceinline__ ZetaTerm<V> zeta_term(V rx, V ry, V rz, V sj) {
+  const V r2 = fma(rx, rx, fma(ry, ry, rz * rz));
+  const V s2 = sj * sj;
+  const V y = rsqrt_lane<REFINE>(r2 + s2);
+  const V y2 = y * y;
+  const V y3 = y2 * y;
+  const V y7 = (y3 * y3) * y;
+  return ZetaTerm<V>{r2, (s2 * s2) * y7};
+}
 
 // ---- probe vorticity (zeta kernel only): W += s^4 y^7 a_j, r^2 <= 1e-8 skipped ----------
 template <class V, bool REFINE>
 struct OpVortAt : PairOpBase<V> {
+  static constexpr int kR = kProbeR<V>;
   static constexpr int NV = 3;
+  static constexpr bool kGuarded = true;
+  static constexpr int kGuardGroup = LaneTraits<V>::kLanes == 1 ? 4 : 2;
+  using Term = ZetaTerm<V>;
+  __device__ __forceinline__ static Term term(const Tgt<V>& t, const Src<V>& s) {
+    return zeta_term<V, REFINE>(t.x - s.x, t.y - s.y, t.z - s.z, s.s);
+  }
+  __device__ __forceinline__ static void add(V* acc, const Term& q, const Src<V>& s) {
+    acc[0] = fma(q.k, s.ax, acc[0]);
+    acc[1] = fma(q.k, s.ay, acc[1]);
+    acc[2] = fma(q.k, s.az, acc[2]);
+  }
+  __device__ __forceinline__ static void add_guarded(V* acc, const Term& q, const Src<V>& s) {
+    acc[0] = fma_if_gt(q.r2, kRefEps, q.k, s.ax, acc[0]);
+    acc[1] = fma_if_gt(q.r2, kRefEps, q.k, s.ay, acc[1]);
+    acc[2] = fma_if_gt(q.r2, kRefEps, q.k, s.az, acc[2]);
+  }
   __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
                                               const int64_t*, int64_t) {
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    const V r2 = fma(rx, rx, fma(ry, ry, rz * rz));
-    const V s2 = s.s * s.s;
-    const V y = rsqrt_lane<REFINE>(r2 + s2);
-    const V y2 = y * y;
-    const V y3 = y2 * y;
-    const V y7 = (y3 * y3) * y;
-    const V k = (s2 * s2) * y7;
-    acc[0] = fma_if_gt(r2, kRefEps, k, s.ax, acc[0]);
-    acc[1] = fma_if_gt(r2, kRefEps, k, s.ay, acc[1]);
-    acc[2] = fma_if_gt(r2, kRefEps, k, s.az, acc[2]);
+    add_guarded(acc, term(t, s), s);
   }
 };
 
@@ -234,28 +285,36 @@ __device__ __forceinline__ TgtF<float2> make_tgtf(const RecF<float2>* const* r) 
 template <class V, bool REFINE>
 struct OpTestFilter {
   static constexpr int NV = 5;
-  static constexpr int kR = 0;
+  static constexpr int kR = kProbeR<V>;
   static constexpr int kWindow = 0;
+  static constexpr bool kGuarded = true;
+  static constexpr int kGuardGroup = 4;
   using Record = RecF<V>;
   using SrcT = SrcF<V>;
   using TgtT = TgtF<V>;
+  using Term = ZetaTerm<V>;
   __device__ __forceinline__ static SrcT load(const Record& r) { return load_srcf(r); }
   __device__ __forceinline__ static TgtT target(const Record* const* r) { return make_tgtf(r); }
+  __device__ __forceinline__ static Term term(const TgtT& t, const SrcT& s) {
+    return zeta_term<V, REFINE>(t.x - s.x, t.y - s.y, t.z - s.z, s.s);
+  }
+  __device__ __forceinline__ static void add(V* acc, const Term& q, const SrcT& s) {
+    acc[0] = fma(q.k, s.ax, acc[0]);
+    acc[1] = fma(q.k, s.ay, acc[1]);
+    acc[2] = fma(q.k, s.az, acc[2]);
+    acc[3] = fma(q.k, s.f1, acc[3]);
+    acc[4] = fma(q.k, s.f2, acc[4]);
+  }
+  __device__ __forceinline__ static void add_guarded(V* acc, const Term& q, const SrcT& s) {
+    acc[0] = fma_if_gt(q.r2, kRefEps, q.k, s.ax, acc[0]);
+    acc[1] = fma_if_gt(q.r2, kRefEps, q.k, s.ay, acc[1]);
+    acc[2] = fma_if_gt(q.r2, kRefEps, q.k, s.az, acc[2]);
+    acc[3] = fma_if_gt(q.r2, kRefEps, q.k, s.f1, acc[3]);
+    acc[4] = fma_if_gt(q.r2, kRefEps, q.k, s.f2, acc[4]);
+  }
   __device__ __forceinline__ static void pair(const TgtT& t, V* acc, const SrcT& s,
                                               const int64_t*, int64_t) {
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    const V r2 = fma(rx, rx, fma(ry, ry, rz * rz));
-    const V s2 = s.s * s.s;
-    const V y = rsqrt_lane<REFINE>(r2 + s2);
-    const V y2 = y * y;
-    const V y3 = y2 * y;
-    const V y7 = (y3 * y3) * y;
-    const V k = (s2 * s2) * y7;
-    acc[0] = fma_if_gt(r2, kRefEps, k, s.ax, acc[0]);
-    acc[1] = fma_if_gt(r2, kRefEps, k, s.ay, acc[1]);
-    acc[2] = fma_if_gt(r2, kRefEps, k, s.az, acc[2]);
-    acc[3] = fma_if_gt(r2, kRefEps, k, s.f1, acc[3]);
-    acc[4] = fma_if_gt(r2, kRefEps, k, s.f2, acc[4]);
+    add_guarded(acc, term(t, s), s);
   }
 };
 

@@ -143,8 +143,39 @@ sweep_kernel(const SweepArgs<typename Op::Record> a) {
     if (ok) {
       for (int w = 0; w < cnt; w += CW) {
         const int e = (w + CW < cnt) ? w + CW : cnt;
+        int j = w;
+        if constexpr (Op::kGuarded) {
+          constexpr int kGuardGroup = Op::kGuardGroup;
+          // a few sources at a time: their terms, one test over all their pairs, and the
+          // plain sums unless a pair is (or may be) within the guard radius of its target
+          for (; j + kGuardGroup <= e; j += kGuardGroup) {
+            typename Op::SrcT src[kGuardGroup];
+            typename Op::Term q[kGuardGroup][P];
+            bool clear = true;
+#pragma unroll
+            for (int g = 0; g < kGuardGroup; ++g) {
+              src[g] = Op::load(tile[j + g]);
+#pragma unroll
+              for (int p = 0; p < P; ++p) {
+                q[g][p] = Op::term(tg[p], src[g]);
+                clear &= surely_gt(q[g][p].r2, kRefEps);
+              }
+            }
+            if (clear) {
+#pragma unroll
+              for (int g = 0; g < kGuardGroup; ++g)
+#pragma unroll
+                for (int p = 0; p < P; ++p) Op::add(acc[p], q[g][p], src[g]);
+            } else {
+#pragma unroll
+              for (int g = 0; g < kGuardGroup; ++g)
+#pragma unroll
+                for (int p = 0; p < P; ++p) Op::add_guarded(acc[p], q[g][p], src[g]);
+            }
+          }
+        }
 #pragma unroll kSrcUnroll
-        for (int j = w; j < e; ++j) {
+        for (; j < e; ++j) {
           const typename Op::SrcT src = Op::load(tile[j]);
 #pragma unroll
           for (int p = 0; p < P; ++p) Op::pair(tg[p], acc[p], src, &gi[p * L], jt + j);
