@@ -161,12 +161,13 @@ int vpm_velocity_and_strength_gradients(const double* positions, const double* s
  * alone, PSE and the LES step (vpm_velocity_and_strength_gradients, vpm_selfinduced_velocity,
  * vpm_strength_gradients_pse, vpm_les_step_sums, vpm_rhs_vjp, and vpm_sweep_records over all
  * records) with n >= this value evaluate each unordered pair once for both particles
- * (deterministic tile-pair schedule, about n / (2 T m) launches for tiles of T = 512 or 768
- * particles and m diagonal pairs per launch).  Where those launches are short (up to ~150000
- * particles), the diagonal tiles run on a second stream of the library's, forked from and
- * joined to the caller's stream by events inside the call, so stream order and CUDA-graph
- * capture see one call as before; that stream is created by the first such call in a context
- * (make it before any stream capture).  The FP64 self sums (those above, the stretching and
+ * (deterministic tile-pair schedule).  While the partial sums of a triangle of tile pairs fit
+ * 2 GB (up to 70000 to 400000 particles, by operator and precision) that is one launch beside the
+ * diagonal tiles'; past it about n / (2 T m) launches for tiles of T = 512 or 768 particles and m
+ * diagonal pairs per launch.  The diagonal tiles of the triangle, and of short launches, run on a
+ * second stream of the library's, forked from and joined to the caller's stream by events inside
+ * the call, so stream order and CUDA-graph capture see one call as before; that stream is created
+ * by the first such call in a context (make it before any stream capture).  The FP64 self sums (those above, the stretching and
  * the adjoint among them) do so from a sixth of this value on, in one launch over a circle of
  * tiles; the stretching and the adjoint stay there while their partial sums fit 4 GB.  The scalar
  * diagnostics in FP64 take each unordered pair once at every size.  Sets the threshold and

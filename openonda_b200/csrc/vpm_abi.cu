@@ -24,6 +24,7 @@
 #include "vpm_adjoint.cuh"
 #include "vpm_rot.cuh"
 #include "vpm_circle.cuh"
+#include "vpm_triangle.cuh"
 #include "vpm_sets.cuh"
 #include "vpm_scalar.cuh"
 #include "vpm_small.cuh"
@@ -104,6 +105,8 @@ struct Plan {
   // both-sides sweep: the diagonal tiles run beside the (single) diagonal-pair launch on a
   // second stream, into their own accumulator sets after the pairs' ones
   int diag_beside = 0;
+  // both-sides sweep over a triangle of tile pairs: its sets of target sums; 0 = no
+  int triangle = 0;
   Shares shares{};  // of the one-launch schedules
   int circle = 0;  // FP64 both-sides sweep in one launch (vpm_circle.cuh)
   int small = 0;   // one launch from the caller's arrays (vpm_small.cuh); records: one-sided
@@ -957,6 +960,119 @@ __global__ void finalize_kegrad_kernel(const double* __restrict__ part, int spli
   gsig[i] = 0.5 * c * v[6];
 }
 
+// ---- both-sides sweep over a triangle of tile pairs (vpm_triangle.cuh, vpm_circle.cuh) --------
+// Its partial sums may take this much; past it the sweep is the many-launch one (vpm_rot.cuh),
+// whose accumulators do not grow with n^2.
+constexpr size_t kMaxTriangleBytes = size_t(2) << 30;
+
+template <class Op>
+struct TriSweep {
+  static constexpr int NV = Op::NV;
+  static constexpr int kTile = rot_tile<Op>();
+  static constexpr int kUnit = Op::kFP64 ? 32 : kTriUnit;
+  static constexpr size_t smem() {
+    if constexpr (Op::kFP64)
+      return lists64_smem_bytes<Op>();
+    else
+      return rot_smem_bytes<Op>();
+  }
+  static constexpr size_t kSmem = smem();
+
+  static const void* kernel_ptr() {
+    if constexpr (Op::kFP64)
+      return reinterpret_cast<const void*>(&rot64_lists_kernel<Op, TriLists64>);
+    else
+      return reinterpret_cast<const void*>(&rot_triangle_kernel<Op>);
+  }
+
+  static int prepare(int* occ) {
+    const void* fn = kernel_ptr();
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    const auto key = std::make_pair(fn, dev);
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_occ.find(key);
+    if (it == g_occ.end()) {
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem));
+      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(triangle sweep)");
+      int o = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kRotThreads, kSmem);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+      it = g_occ.emplace(key, o > 0 ? o : 1).first;
+    }
+    *occ = it->second;
+    return VPM_OK;
+  }
+
+  // p: the many-launch plan of the same build.  Sets p->triangle and p->splits where the partial
+  // sums fit; the other fields stay (the pair shards across GPUs use them).
+  static int plan(int64_t n, Plan* p, size_t max_partial_bytes) {
+    DevInfo d;
+    int occ = 1;
+    int rc = device_info(&d);
+    if (!rc) rc = prepare(&occ);
+    if (!rc) rc = RotSweep<Op>::prepare_side();
+    if (rc || n >= (int64_t(1) << 30)) return rc;
+    const TriLists l(n, kTile, kUnit);
+    const Shares shares = Shares::make(l.total(), int64_t(d.sms) * occ);
+    const int tsets = target_sets(l, shares);
+    const int64_t sets =
+        kRotDiagSplit + tsets + (l.before(l.nt - 1, n, kTile) + n - 1) / n;
+    const size_t bytes = size_t(sets) * NV * size_t(n) * sizeof(double);
+    if (bytes > max_partial_bytes || bytes > kMaxTriangleBytes) return VPM_OK;
+    p->triangle = tsets;
+    p->shares = shares;
+    p->splits = int(sets);
+    return VPM_OK;
+  }
+
+  // acc: [p.splits][NV][n]: the diagonal tiles' sets, the target sets, the source sets.  The
+  // diagonal tiles run beside on the side stream, launched first, so that their few blocks are
+  // done when the shares that wait for their places begin.
+  template <class Finalize>
+  static int launch(const Plan& p, const void* rec, int64_t n, double* acc, const Finalize& fin,
+                    cudaStream_t st) {
+    const TriLists l(n, kTile, kUnit);
+    const int tsets = p.triangle;
+    double* target = acc + int64_t(kRotDiagSplit) * NV * n;
+    double* source = target + int64_t(tsets) * NV * n;
+    int rc = zero_out(acc, int64_t(kRotDiagSplit) * NV * n, st);
+    if (!rc) {
+      std::unique_lock<std::mutex> lk(g_side_mu);
+      SideStream* ss = nullptr;
+      rc = side_stream(&ss);
+      if (rc) return rc;
+      cudaError_t e = cudaEventRecord(ss->fork, st);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(ss->stream, ss->fork, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "side stream fork");
+      RotSweep<Op>::template launch_kernel<true>(unsigned(l.nt * kRotDiagSplit),
+                                                 RotArgs{rec, n, l.nt, 0, acc}, ss->stream);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return cuda_fail(e, "both-sides sweep launch");
+      const unsigned grid = unsigned(p.shares.blocks());
+      if constexpr (Op::kFP64) {
+        const Sweep64Args a{rec, int(n), p.shares, target, source};
+        rot64_lists_kernel<Op, TriLists64><<<grid, kRotThreads, kSmem, st>>>(a);
+      } else {
+        const TriArgs a{rec, int(n), l.nt, p.shares, target, source};
+        rot_triangle_kernel<Op><<<grid, kRotThreads, kSmem, st>>>(a);
+      }
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return cuda_fail(e, "triangle sweep launch");
+      e = cudaEventRecord(ss->join, ss->stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ss->join, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "side stream join");
+    }
+    if (rc) return rc;
+    const TriSets sets{l, p.shares, kTile, kRotDiagSplit, n, source};
+    finalize_sets_kernel<NV, Op::kSymFrom, TriSets, Finalize>
+        <<<unsigned((n + 31) / 32), 32 * kSetLanes, 0, st>>>(acc, sets, n, fin);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
+  }
+};
+
 // ---- FP64 both-sides sweep in one launch (vpm_circle.cuh) ------------------------------------
 // Lower end of its range, a sixth of the both-sides threshold (so that vpm_set_symmetric_min_n
 // moves both): 4096 particles by default.  Measured against the one-sided sweeps (us, velocity /
@@ -1035,8 +1151,8 @@ struct CircleSweep {
 
 
 // The FP64 plan of a self sum of n particles on the both-sides schedules, if it takes one
-// (p->circle or p->pairs set).  MULTI: from the threshold on the sum takes the many-launch sweep;
-// otherwise the circle at all sizes its sets fit.
+// (p->circle or p->pairs set).  MULTI: from the threshold on the sum takes the triangle, and the
+// many-launch sweep past the triangle's budget; otherwise the circle at all sizes its sets fit.
 template <class Op, bool MULTI>
 int plan_both64(int64_t m, int64_t n, Plan* p, size_t mpb) {
   if (m != n) return VPM_OK;
@@ -1046,7 +1162,19 @@ int plan_both64(int64_t m, int64_t n, Plan* p, size_t mpb) {
     int rc = CircleSweep<Op>::plan(n, p, mpb);
     if (rc || p->circle) return rc;
   }
-  return large ? RotSweep<Op>::plan(n, p, mpb) : VPM_OK;
+  if (!large) return VPM_OK;
+  int rc = RotSweep<Op>::plan(n, p, mpb);
+  if (!rc && MULTI) rc = TriSweep<Op>::plan(n, p, mpb);
+  return rc;
+}
+
+// The FP32 both-sides plan of a self sum: the many-launch sweep's, and the one-launch form where
+// its partial sums fit.
+template <class Op>
+int plan_both32(int64_t n, Plan* p, size_t mpb) {
+  int rc = RotSweep<Op>::plan(n, p, mpb);
+  if (!rc) rc = TriSweep<Op>::plan(n, p, mpb);
+  return rc;
 }
 
 // ---- small sums in one launch (vpm_small.cuh) ---------------------------------------------
@@ -1193,7 +1321,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
     case VPM_OP_SELFINDUCED_VELOCITY:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::VelBoth>::usable(m, n, mpb))
-          return RotSweep<typename O::VelBoth>::plan(n, p, mpb);
+          return plan_both32<typename O::VelBoth>(n, p, mpb);
       } else {
         const int rc = plan_both64<typename O::VelBoth64, true>(m, n, p, mpb);
         if (rc || p->circle || p->pairs) return rc;
@@ -1217,7 +1345,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
     case VPM_OP_STRENGTH_GRADIENTS_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::PseBoth>::usable(m, n, mpb))
-          return RotSweep<typename O::PseBoth>::plan(n, p, mpb);
+          return plan_both32<typename O::PseBoth>(n, p, mpb);
       } else {
         const int rc = plan_both64<typename O::PseBoth64, true>(m, n, p, mpb);
         if (rc || p->circle || p->pairs) return rc;
@@ -1265,7 +1393,10 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
               *p = pc;
             }
           }
-          return VPM_OK;
+          // the one-launch form of the same tiles (the same FP32 sums); of the two builds on
+          // 768-particle tiles the one for 2 CTAs per SM
+          return p->variant == 2 ? TriSweep<typename O::VelStretchBothSmall>::plan(n, p, mpb)
+                                 : TriSweep<typename O::VelStretchBothAlt>::plan(n, p, mpb);
         }
       } else {
         const int rc = plan_both64<typename O::VelStretchBoth64, true>(m, n, p, mpb);
@@ -1275,7 +1406,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
     case VPM_OP_LES_STEP_SUMS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::LesStepBoth>::usable(m, n, mpb))
-          return RotSweep<typename O::LesStepBoth>::plan(n, p, mpb);
+          return plan_both32<typename O::LesStepBoth>(n, p, mpb);
       } else {
         const int rc = plan_both64<typename O::LesStepBoth64, true>(m, n, p, mpb);
         if (rc || p->circle || p->pairs) return rc;
@@ -1284,7 +1415,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
     case VPM_OP_RHS_VJP:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::RhsVjpBoth>::usable(m, n, mpb))
-          return RotSweep<typename O::RhsVjpBoth>::plan(n, p, mpb);
+          return plan_both32<typename O::RhsVjpBoth>(n, p, mpb);
       } else {
         const int rc = plan_both64<typename O::RhsVjpBoth64, false>(m, n, p, mpb);
         if (rc || p->circle || p->pairs) return rc;
@@ -1293,7 +1424,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
     case VPM_OP_RHS_VJP_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::RhsVjpPseBoth>::usable(m, n, mpb))
-          return RotSweep<typename O::RhsVjpPseBoth>::plan(n, p, mpb);
+          return plan_both32<typename O::RhsVjpPseBoth>(n, p, mpb);
       } else {
         const int rc = plan_both64<typename O::RhsVjpPseBoth64, false>(m, n, p, mpb);
         if (rc || p->circle || p->pairs) return rc;
@@ -1443,6 +1574,14 @@ int run(const Call& c) {
           return CircleSweep<typename O::VelBoth64>::launch(
               p, src, c.n, part, SetsFinalize<double, FIN_VEL, 3>{src, c.out, nullptr, nullptr, nullptr},
               c.st);
+        if (p.triangle)
+          return TriSweep<typename O::VelBoth64>::launch(
+              p, src, c.n, part, SetsFinalize<double, FIN_VEL, 3>{src, c.out, nullptr, nullptr, nullptr},
+              c.st);
+      } else if (p.triangle) {
+        return TriSweep<typename O::VelBoth>::launch(
+            p, src, c.n, part, SetsFinalize<T, FIN_VEL, 3>{src, c.out, nullptr, nullptr, nullptr},
+            c.st);
       }
       if (p.pairs) {  // m == n: the targets are all the records (tgt_begin == 0)
         if constexpr (LaneTraits<T>::kLanes == 2)
@@ -1483,6 +1622,14 @@ int run(const Call& c) {
           return CircleSweep<typename O::PseBoth64>::launch(
               p, src, c.n, part, SetsFinalize<double, FIN_PSE, 3>{src, c.out, nullptr, nullptr, nullptr},
               c.st);
+        if (p.triangle)
+          return TriSweep<typename O::PseBoth64>::launch(
+              p, src, c.n, part, SetsFinalize<double, FIN_PSE, 3>{src, c.out, nullptr, nullptr, nullptr},
+              c.st);
+      } else if (p.triangle) {
+        return TriSweep<typename O::PseBoth>::launch(
+            p, src, c.n, part, SetsFinalize<T, FIN_PSE, 3>{src, c.out, nullptr, nullptr, nullptr},
+            c.st);
       }
       if (p.pairs) {
         if constexpr (LaneTraits<T>::kLanes == 2)
@@ -1496,6 +1643,12 @@ int run(const Call& c) {
       return rc;
     case VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
+        if (p.triangle) {
+          const SetsFinalize<T, FIN_VELSTRETCH, 9> fin{src, c.out, c.out2, nullptr, nullptr};
+          if (p.variant == 2)
+            return TriSweep<typename O::VelStretchBothSmall>::launch(p, src, c.n, part, fin, c.st);
+          return TriSweep<typename O::VelStretchBothAlt>::launch(p, src, c.n, part, fin, c.st);
+        }
         if (p.pairs && p.variant == 2)  // m == n: the targets are all the records
           rc = RotSweep<typename O::VelStretchBothSmall>::launch(p, src, c.n, part, c.st);
         else if (p.pairs && p.variant == 1)
@@ -1507,6 +1660,10 @@ int run(const Call& c) {
                                                         part, c.st);
       } else if (p.circle) {
         return CircleSweep<typename O::VelStretchBoth64>::launch(
+            p, src, c.n, part,
+            SetsFinalize<double, FIN_VELSTRETCH, 9>{src, c.out, c.out2, nullptr, nullptr}, c.st);
+      } else if (p.triangle) {
+        return TriSweep<typename O::VelStretchBoth64>::launch(
             p, src, c.n, part,
             SetsFinalize<double, FIN_VELSTRETCH, 9>{src, c.out, c.out2, nullptr, nullptr}, c.st);
       } else if (p.pairs) {
@@ -1522,7 +1679,7 @@ int run(const Call& c) {
     case VPM_OP_LES_STEP_SUMS: {
       using Op = typename O::LesStep;
       rc = VPM_OK;
-      if (p.pairs) {
+      if (p.pairs && !p.triangle) {
         if constexpr (LaneTraits<T>::kLanes == 2)
           rc = RotSweep<typename O::LesStepBoth>::launch(p, src, c.n, part, c.st);
         else
@@ -1545,6 +1702,19 @@ int run(const Call& c) {
           scale *= 2.0;
           done = true;
         }
+        if (p.triangle) {
+          rc = TriSweep<typename O::LesStepBoth64>::launch(
+              p, src, c.n, part,
+              SetsFinalize<double, FIN_LES, NVB>{src, c.out, c.out2, c.out3, scalar}, c.st);
+          scale *= 2.0;
+          done = true;
+        }
+      } else if (p.triangle) {
+        rc = TriSweep<typename O::LesStepBoth>::launch(
+            p, src, c.n, part,
+            SetsFinalize<T, FIN_LES, NVB>{src, c.out, c.out2, c.out3, scalar}, c.st);
+        scale *= 2.0;
+        done = true;
       }
       if (!done && p.pairs) {
         rc = finalize_vec<T, FIN_LES, NVB>(part, p.splits, c.m, tgt, c.out, c.out2, c.st, c.out3,
@@ -1765,6 +1935,9 @@ int run_grad(const GradCall& c) {
   if (c.op == VPM_OP_RHS_VJP_PSE) {
     rc = VPM_OK;
     if constexpr (LaneTraits<T>::kLanes == 2) {
+      if (p.triangle)
+        return TriSweep<typename O::RhsVjpPseBoth>::launch(
+            p, rec, c.n, part, SetsFinalizeVjp<T, true>{rec, c.ox, c.oa, c.os, c.onu}, c.st);
       if (p.pairs) rc = RotSweep<typename O::RhsVjpPseBoth>::launch(p, rec, c.n, part, c.st);
     } else {
       if (p.circle)
@@ -1780,6 +1953,9 @@ int run_grad(const GradCall& c) {
   } else {
     rc = VPM_OK;
     if constexpr (LaneTraits<T>::kLanes == 2) {
+      if (p.triangle)
+        return TriSweep<typename O::RhsVjpBoth>::launch(
+            p, rec, c.n, part, SetsFinalizeVjp<T, false>{rec, c.ox, c.oa, c.os, c.onu}, c.st);
       if (p.pairs) rc = RotSweep<typename O::RhsVjpBoth>::launch(p, rec, c.n, part, c.st);
     } else {
       if (p.circle)
@@ -2259,6 +2435,9 @@ int64_t vpm_sweep_launches(int op, int precision, int64_t m, int64_t n) {
     return plan_op<typename Pp::type, Pp::refine, Pp::uc>(op, m, n, &p);
   });
   if (rc) return -1;
+  if (p.triangle) {  // zero the diagonal tiles' sets, those tiles, the triangle, finalize
+    return op == VPM_OP_LES_STEP_SUMS ? 5 : 4;
+  }
   if (p.pairs) {  // zero the accumulators, the diagonal tiles, the diagonal-pair launches, finalize
     const int64_t npairs = p.tblocks / 2;
     return 3 + (npairs + p.pairs - 1) / p.pairs;

@@ -47,6 +47,7 @@ struct Sweep64Args {
 
 // The lists: target tile I's has (1 + distances) tiles of `per` batches, its own tile first.
 struct CircleLists {
+  static constexpr bool kOwnTile = true;
   int nt, half, per;
   __host__ __device__ CircleLists(int64_t n, int tile) {
     nt = int((n + tile - 1) / tile);
@@ -77,6 +78,19 @@ struct CircleLists {
     const int64_t first = start(full());
     if (w < first) return int(w / (int64_t(1 + half) * per));
     return full() + int((w - first) / (int64_t(half) * per));
+  }
+};
+
+// The triangle of vpm_shares.cuh in the same form (batches of 32): every tile pair with the lower
+// tile as target, the diagonal tiles left to rot64_sweep_kernel<Op, true>.
+struct TriLists64 : TriLists {
+  static constexpr bool kOwnTile = false;
+  __host__ __device__ TriLists64(int64_t n, int tile) : TriLists(n, tile, 32) {}
+  __device__ __forceinline__ int source_tile(int I, int t) const { return I + 1 + t; }
+  __device__ __forceinline__ double* source_sums(double* source, int nv, int I, int, int j,
+                                                 int64_t n, int tile, int64_t& stride) const {
+    stride = n - int64_t(I + 1) * tile;
+    return source + int64_t(nv) * before(I, n, tile) + j - int64_t(I + 1) * tile;
   }
 };
 
@@ -157,7 +171,7 @@ rot64_lists_kernel(const Sweep64Args a) {
         cnt = place(b + 1, j0);
         if (Op::kPrefetch) nxt = Op::load(rec, j0 + lane, j0 + cnt);
       }
-      if (b < PER) {  // the tile's own sources, one-sided
+      if (Lists::kOwnTile && b < PER) {  // the tile's own sources, one-sided
 #pragma unroll 1
         for (int st = 0; st < 32; ++st) {
 #pragma unroll

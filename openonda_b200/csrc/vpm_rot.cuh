@@ -798,15 +798,53 @@ __device__ __forceinline__ bool rot_block_pair(const RotArgs& a, int& I, int& J,
   return false;  // k == nt - k: the diagonal has only nt - k tile pairs
 }
 
+// The target rows of a thread: packed lane p holds warp * 64 P + 64 p + lane + {0, 32}.
+template <int P>
+__device__ __forceinline__ void rot_rows(int (&lt)[2 * P], int warp, int lane) {
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+    lt[2 * p] = warp * 64 * P + p * 64 + lane;
+    lt[2 * p + 1] = lt[2 * p] + 32;
+  }
+}
+
+// Target side: the FP32 window sums of the values take(v) selects into the FP64 carries
+// car[NV][T] (each thread its own rows), and those sums start again from zero.
+template <class Op, bool DIAG, class Take>
+__device__ __forceinline__ void rot_fold(double* car, float2 (&acc)[Op::kP][Op::NV],
+                                         const int (&lt)[2 * Op::kP], Take&& take) {
+  constexpr int T = rot_tile<Op>();
+#pragma unroll
+  for (int p = 0; p < Op::kP; ++p) {
+#pragma unroll
+    for (int v = 0; v < Op::NV; ++v) {
+      if (!take(v)) continue;
+      if (DIAG && v >= Op::kSymFrom) {
+        // a symmetric sum taken once per unordered pair elsewhere: the diagonal tiles visit
+        // every ordered pair, so they count half (the finalize doubles the sum)
+        car[v * T + lt[2 * p]] += 0.5 * double(acc[p][v].x);
+        car[v * T + lt[2 * p + 1]] += 0.5 * double(acc[p][v].y);
+      } else {
+        car[v * T + lt[2 * p]] += double(acc[p][v].x);
+        car[v * T + lt[2 * p + 1]] += double(acc[p][v].y);
+      }
+      acc[p][v] = make_float2(0.f, 0.f);
+    }
+  }
+}
+
+// Batch b of a source tile (sources j .. j + 31, lane l holding source j + l at step 0) against
+// the warp's targets; i0: the target tile's first particle.  The warp's packed source-side sums
+// go to its slots of jb, [kSymFrom][warps * 32].
 template <class Op, bool DIAG>
-__global__ void __launch_bounds__(kRotThreads, Op::kMinBlocks)
-rot_sweep_kernel(const RotArgs a) {
-  using Record = typename Op::Record;
-  using Lane = typename Op::Lane;
+__device__ __forceinline__ void rot_batch(typename Op::Lane cur,
+                                          const typename Op::TgtT (&tg)[Op::kP],
+                                          float2 (&acc)[Op::kP][Op::NV],
+                                          const int (&lt)[2 * Op::kP], double* car, float2* jb,
+                                          int64_t i0, int64_t j, int b, int warp, int lane) {
   constexpr int NV = Op::NV;
   constexpr int P = Op::kP;
-  constexpr int T = rot_tile<Op>();
-  constexpr int WT = kRotWarps * 32;  // source slots of a batch: [warp][source lane]
+  constexpr int WT = kRotWarps * 32;
   constexpr int SW = Op::kSrcWindow;
   constexpr int TW = Op::kTgtWindow;
   static_assert(32 % SW == 0, "the source window divides the 32 steps of a batch");
@@ -816,10 +854,99 @@ rot_sweep_kernel(const RotArgs a) {
                 "short target windows divide the target window and are whole source windows");
   constexpr int TWL = Op::kTgtWindowLong;
   static_assert(TWL == 0 || TWL % 32 == 0, "long target windows are whole batches");
+  float2 jv[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) jv[v] = make_float2(0.f, 0.f);
+  const int src_lane = (lane + 1) & 31;
+  for (int w = 0; w < 32 / SW; ++w) {
+#pragma unroll Op::kUnroll
+    for (int st = 0; st < SW; ++st) {
+      const int step = w * SW + st;
+      const typename Op::SrcT src = Op::broadcast(cur);
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        if constexpr (DIAG) {
+          // at this step the lane holds source (lane + step) mod 32 of the batch
+          const int64_t ti[2] = {i0 + lt[2 * p], i0 + lt[2 * p + 1]};
+          Op::diag(tg[p], acc[p], src, ti, j + ((lane + step) & 31));
+        } else {
+          Op::pair2(tg[p], acc[p], jv, src);
+        }
+      }
+      // pass the source one lane down (lane l now holds what lane l+1 held); its sums move
+      // with it, except after a window's last step, where they are stored instead
+      Op::shuffle(cur, src_lane);
+      if constexpr (!DIAG) {
+        if (st != SW - 1) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            if (Op::carried(v)) {
+              jv[v].x = __shfl_sync(0xffffffffu, jv[v].x, src_lane);
+              jv[v].y = __shfl_sync(0xffffffffu, jv[v].y, src_lane);
+            }
+          }
+        }
+      }
+    }
+    if constexpr (!DIAG) {
+      // end of a window: the lane holds the sums of the source it met at the window's last
+      // step, (lane + step) mod 32; add them into that source's slot (the lanes of a warp
+      // hold distinct sources) and start the next window from zero
+      const int slot = warp * 32 + ((lane + (w + 1) * SW - 1) & 31);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        if (Op::carried(v)) {
+          float2* e = jb + v * WT + slot;
+          *e = (w == 0) ? jv[v] : (*e + jv[v]);
+          jv[v] = make_float2(0.f, 0.f);
+        }
+      }
+    }
+    const int done = (w + 1) * SW;  // steps of this batch done
+    const bool at_full = done % TW == 0;
+    const bool at_short = TWS > 0 && done % (TWS > 0 ? TWS : 1) == 0;
+    const bool at_long = TWL > 0 && (b * 32 + done) % (TWL > 0 ? TWL : 1) == 0;
+    if (at_full || at_short || at_long)
+      rot_fold<Op, DIAG>(car, acc, lt, [&](int v) {
+        return (TWL > 0 && Op::long_fold(v))    ? at_long
+               : (TWS > 0 && Op::short_fold(v)) ? at_short
+                                                : at_full;
+      });
+  }
+}
+
+// The warps' source-side sums of a batch of nsrc sources (both packed halves of every warp's
+// sum), in FP64 and in a fixed order: store(v, jj, sum) for value v of source jj, the sums with
+// their accumulated (opposite) sign.
+template <class Op, class Store>
+__device__ __forceinline__ void rot_combine(const float2* jb, int nsrc, int tid, Store&& store) {
+  constexpr int WT = kRotWarps * 32;
+  for (int q = tid; q < 32 * Op::kSymFrom; q += kRotThreads) {
+    const int v = q >> 5, jj = q & 31;  // consecutive threads: consecutive sources
+    if (jj >= nsrc || !Op::carried(v)) continue;
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kRotWarps; ++w) {
+      const float2 e = jb[v * WT + w * 32 + jj];
+      sum += double(e.x);
+      sum += double(e.y);
+    }
+    store(v, jj, sum);
+  }
+}
+
+template <class Op, bool DIAG>
+__global__ void __launch_bounds__(kRotThreads, Op::kMinBlocks)
+rot_sweep_kernel(const RotArgs a) {
+  using Record = typename Op::Record;
+  using Lane = typename Op::Lane;
+  constexpr int NV = Op::NV;
+  constexpr int P = Op::kP;
+  constexpr int T = rot_tile<Op>();
+  constexpr int NJ = Op::kSymFrom;  // values with a source side: the first NJ
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* car = reinterpret_cast<double*>(smem_raw);  // [NV][T]
-  // [2][NV][WT]: each warp's packed source-side sums of the current batch, per source
-  constexpr int NJ = Op::kSymFrom;  // values with a source side: the first NJ
+  // [2][NJ][WT]: each warp's packed source-side sums of the current batch, per source
   float2* jbuf = reinterpret_cast<float2*>(smem_raw + size_t(T) * NV * sizeof(double));
   const Record* rec = static_cast<const Record*>(a.rec);
 
@@ -834,13 +961,11 @@ rot_sweep_kernel(const RotArgs a) {
 
   for (int q = tid; q < T * NV; q += kRotThreads) car[q] = 0.0;
 
-  // this lane's targets: packed lane p holds warp * 64P + 64p + lane + {0, 32}
   int lt[2 * P];
+  rot_rows<P>(lt, warp, lane);
   typename Op::TgtT tg[P];
 #pragma unroll
   for (int p = 0; p < P; ++p) {
-    lt[2 * p] = warp * 64 * P + p * 64 + lane;
-    lt[2 * p + 1] = lt[2 * p] + 32;
     const int64_t t0 = i0 + lt[2 * p], t1 = i0 + lt[2 * p + 1];
     // targets past n (a copy of the last record) occur only in the diagonal tiles: a tile
     // pair has I < J <= nt - 1, so its target tile is whole; the diagonal tiles are one-sided,
@@ -856,117 +981,27 @@ rot_sweep_kernel(const RotArgs a) {
     for (int v = 0; v < NV; ++v) acc[p][v] = make_float2(0.f, 0.f);
   __syncthreads();  // carries zeroed
 
-  // target side: the FP32 window sums of the values take(v) selects into the FP64 carries
-  // (each thread its own rows), and those sums start again from zero
-  auto fold_targets = [&](auto take) {
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        if (!take(v)) continue;
-        if (DIAG && v >= NJ) {
-          // a symmetric sum taken once per unordered pair elsewhere: the diagonal tiles
-          // visit every ordered pair, so they count half (the finalize doubles the sum)
-          car[v * T + lt[2 * p]] += 0.5 * double(acc[p][v].x);
-          car[v * T + lt[2 * p + 1]] += 0.5 * double(acc[p][v].y);
-        } else {
-          car[v * T + lt[2 * p]] += double(acc[p][v].x);
-          car[v * T + lt[2 * p + 1]] += double(acc[p][v].y);
-        }
-        acc[p][v] = make_float2(0.f, 0.f);
-      }
-    }
-  };
-
   const int nb = (cnt + 31) / 32;
   Lane nxt = Op::load_lane(rec, j0 + lane, j0 + cnt);
   for (int b = 0; b < nb; ++b) {
-    Lane cur = nxt;  // the source this lane holds at step 0
+    const Lane cur = nxt;  // the source this lane holds at step 0
     if (b + 1 < nb) nxt = Op::load_lane(rec, j0 + (b + 1) * 32 + lane, j0 + cnt);
-    float2 jv[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) jv[v] = make_float2(0.f, 0.f);
-    float2* jb = jbuf + (b % Op::kJBufs) * (NJ * WT);
-    const int src_lane = (lane + 1) & 31;
-    for (int w = 0; w < 32 / SW; ++w) {
-#pragma unroll Op::kUnroll
-      for (int st = 0; st < SW; ++st) {
-        const int step = w * SW + st;
-        const typename Op::SrcT src = Op::broadcast(cur);
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-          if constexpr (DIAG) {
-            // at this step the lane holds source b * 32 + ((lane + step) mod 32) of the tile
-            const int64_t ti[2] = {i0 + lt[2 * p], i0 + lt[2 * p + 1]};
-            Op::diag(tg[p], acc[p], src, ti, j0 + b * 32 + ((lane + step) & 31));
-          } else {
-            Op::pair2(tg[p], acc[p], jv, src);
-          }
-        }
-        // pass the source one lane down (lane l now holds what lane l+1 held); its sums move
-        // with it, except after a window's last step, where they are stored instead
-        Op::shuffle(cur, src_lane);
-        if constexpr (!DIAG) {
-          if (st != SW - 1) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-              if (Op::carried(v)) {
-                jv[v].x = __shfl_sync(0xffffffffu, jv[v].x, src_lane);
-                jv[v].y = __shfl_sync(0xffffffffu, jv[v].y, src_lane);
-              }
-            }
-          }
-        }
-      }
-      if constexpr (!DIAG) {
-        // end of a window: the lane holds the sums of the source it met at the window's last
-        // step, (lane + step) mod 32; add them into that source's slot (the lanes of a warp
-        // hold distinct sources) and start the next window from zero
-        const int slot = warp * 32 + ((lane + (w + 1) * SW - 1) & 31);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          if (Op::carried(v)) {
-            float2* e = jb + v * WT + slot;
-            *e = (w == 0) ? jv[v] : (*e + jv[v]);
-            jv[v] = make_float2(0.f, 0.f);
-          }
-        }
-      }
-      const int done = (w + 1) * SW;  // steps of this batch done
-      const bool at_full = done % TW == 0;
-      const bool at_short = TWS > 0 && done % (TWS > 0 ? TWS : 1) == 0;
-      const bool at_long = TWL > 0 && (b * 32 + done) % (TWL > 0 ? TWL : 1) == 0;
-      if (at_full || at_short || at_long)
-        fold_targets([&](int v) {
-          return (TWL > 0 && Op::long_fold(v))    ? at_long
-                 : (TWS > 0 && Op::short_fold(v)) ? at_short
-                                                  : at_full;
-        });
-    }
+    float2* jb = jbuf + (b % Op::kJBufs) * (NJ * kRotWarps * 32);
+    rot_batch<Op, DIAG>(cur, tg, acc, lt, car, jb, i0, j0 + b * 32, b, warp, lane);
     if constexpr (!DIAG) {
       __syncthreads();  // the batch's source-side sums are complete
-      const int nsrc = (cnt - b * 32 < 32) ? cnt - b * 32 : 32;
-      for (int q = tid; q < 32 * NJ; q += kRotThreads) {
-        const int v = q >> 5, jj = q & 31;  // consecutive threads: consecutive sources
-        if (jj >= nsrc || !Op::carried(v)) continue;
-        // both packed halves of every warp's sum, in FP64, in a fixed order
-        double sum = 0.0;
-#pragma unroll
-        for (int w = 0; w < kRotWarps; ++w) {
-          const float2 e = jb[v * WT + w * 32 + jj];
-          sum += double(e.x);
-          sum += double(e.y);
-        }
+      rot_combine<Op>(jb, cnt - b * 32, tid, [&](int v, int jj, double sum) {
         // the only writer of this element in this launch, so the fire-and-forget reduction
         // adds in a fixed order (launch order) and the thread does not wait for the load
         atomicAdd(&a.acc[(int64_t(set_j) * NV + v) * a.n + (j0 + b * 32 + jj)], -sum);
-      }
+      });
       // one buffer: every thread has read it before the next batch writes it
       if constexpr (Op::kJBufs == 1) __syncthreads();
     }
   }
   // long windows span batches: what the last one left
-  if constexpr (TWL > 0) fold_targets([](int v) { return Op::long_fold(v); });
+  if constexpr (Op::kTgtWindowLong > 0)
+    rot_fold<Op, DIAG>(car, acc, lt, [](int v) { return Op::long_fold(v); });
   __syncthreads();
   for (int q = tid; q < T * NV; q += kRotThreads) {
     const int v = q / T, t = q - v * T;
