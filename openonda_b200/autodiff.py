@@ -116,16 +116,25 @@ def kinetic_energy(x, a, sigma, precision="fp64"):
     return KineticEnergy.apply(x, a, sigma, precision)
 
 
+def _axpy(x, k, c):
+    """x + c k in one operation where c is a plain number (a tensor c keeps its gradient)."""
+    return torch.add(x, k, alpha=c) if isinstance(c, (int, float)) else x + c * k
+
+
+def _rk4_combine(x, k1, k2, k3, k4, dt):
+    s = torch.add(torch.add(k1, k2, alpha=2), k3, alpha=2) + k4
+    return _axpy(x, s, dt / 6)
+
+
 def rk4_step(x, a, sigma, nu, dt, precision="fp64", uniform_core=False):
     """One classical RK4 step of (x, alpha) with frozen sigma and nu."""
     uc = uniform_core
     k1x, k1a = rhs(x, a, sigma, nu, precision, uc)
-    k2x, k2a = rhs(x + (dt / 2) * k1x, a + (dt / 2) * k1a, sigma, nu, precision, uc)
-    k3x, k3a = rhs(x + (dt / 2) * k2x, a + (dt / 2) * k2a, sigma, nu, precision, uc)
-    k4x, k4a = rhs(x + dt * k3x, a + dt * k3a, sigma, nu, precision, uc)
-    x1 = x + (dt / 6) * (k1x + 2 * k2x + 2 * k3x + k4x)
-    a1 = a + (dt / 6) * (k1a + 2 * k2a + 2 * k3a + k4a)
-    return x1, a1
+    k2x, k2a = rhs(_axpy(x, k1x, dt / 2), _axpy(a, k1a, dt / 2), sigma, nu, precision, uc)
+    k3x, k3a = rhs(_axpy(x, k2x, dt / 2), _axpy(a, k2a, dt / 2), sigma, nu, precision, uc)
+    k4x, k4a = rhs(_axpy(x, k3x, dt), _axpy(a, k3a, dt), sigma, nu, precision, uc)
+    return (_rk4_combine(x, k1x, k2x, k3x, k4x, dt),
+            _rk4_combine(a, k1a, k2a, k3a, k4a, dt))
 
 
 def trajectory(x0, a0, sigma, nu=None, dt=0.01, steps=10, precision="fp64",

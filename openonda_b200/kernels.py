@@ -29,6 +29,9 @@ _F64 = torch.float64
 
 
 def _check_vec(name, t, n=None):
+    if (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is _F64 and t.dim() == 2
+            and t.shape[1] == 3 and (n is None or t.shape[0] == n)):
+        return t.contiguous()
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if t.device.type != "cuda":
@@ -43,6 +46,9 @@ def _check_vec(name, t, n=None):
 
 
 def _check_scalar(name, t, n):
+    if (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is _F64 and t.dim() == 1
+            and t.shape[0] == n):
+        return t.contiguous()
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if t.device.type != "cuda":
@@ -68,7 +74,9 @@ def _ptr(t):
 
 
 def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
+    # the handle alone: torch.cuda.current_stream() builds a Stream object around it first
+    return torch._C._cuda_getCurrentRawStream(
+        torch.cuda.current_device() if dev.index is None else dev.index)
 
 
 def workspace_bytes(op: str, precision: str, m: int, n: int, uniform_core: bool = False) -> int:
@@ -99,6 +107,17 @@ def _workspace(op, precision, m, n, dev, uniform_core=False):
     return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev), nbytes
 
 
+def _scratch(op, code, m, n, dev):
+    """Scratch of a sum with the precision code ``code``: (pointer, bytes, tensor)."""
+    nbytes = _lib.load().vpm_workspace_bytes(_lib.OPS[op], code, m, n)
+    if nbytes == 0 and m > 0 and n > 0:
+        msg = _lib.load().vpm_last_error()
+        raise _lib.VPMError(_lib.VPM_ERR_CUDA, msg.decode() if msg else "workspace query failed")
+    nbytes = max(nbytes, 256)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    return ws.data_ptr(), nbytes, ws
+
+
 def _self_inputs(positions, strengths, radii):
     positions = _check_vec("positions", positions)
     n = positions.shape[0]
@@ -108,38 +127,42 @@ def _self_inputs(positions, strengths, radii):
     return positions, strengths, radii, n, dev
 
 
+def _out(x):
+    """A new (n, 3) result like the contiguous positions x."""
+    return torch.empty_like(x)
+
+
 def selfinduced_velocity(positions, strengths, radii, precision="fp64", uniform_core=False):
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
-    out = torch.empty((n, 3), dtype=_F64, device=dev)
-    ws, nb = _workspace("selfinduced_velocity", precision, n, n, dev, uniform_core)
+    out = _out(x)
+    code = _lib.precision_code(precision, uniform_core)
+    ws, nb, _keep = _scratch("selfinduced_velocity", code, n, n, dev)
     _lib.check(_lib.load().vpm_selfinduced_velocity(
-        _ptr(x), _ptr(a), _ptr(s), n, _ptr(out),
-        _lib.precision_code(precision, uniform_core), _ptr(ws),
-        ws.numel(), _stream(dev)))
+        x.data_ptr(), a.data_ptr(), s.data_ptr(), n, out.data_ptr(), code, ws, nb,
+        _stream(dev)))
     return out
 
 
 def strength_gradients(positions, strengths, radii, precision="fp64", uniform_core=False):
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
-    out = torch.empty((n, 3), dtype=_F64, device=dev)
-    ws, nb = _workspace("strength_gradients", precision, n, n, dev, uniform_core)
+    out = _out(x)
+    code = _lib.precision_code(precision, uniform_core)
+    ws, nb, _keep = _scratch("strength_gradients", code, n, n, dev)
     _lib.check(_lib.load().vpm_strength_gradients(
-        _ptr(x), _ptr(a), _ptr(s), n, _ptr(out),
-        _lib.precision_code(precision, uniform_core), _ptr(ws),
-        ws.numel(), _stream(dev)))
+        x.data_ptr(), a.data_ptr(), s.data_ptr(), n, out.data_ptr(), code, ws, nb,
+        _stream(dev)))
     return out
 
 
 def velocity_and_strength_gradients(positions, strengths, radii,
                                     precision="fp64", uniform_core=False):
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
-    u = torch.empty((n, 3), dtype=_F64, device=dev)
-    g = torch.empty((n, 3), dtype=_F64, device=dev)
-    ws, nb = _workspace("velocity_and_strength_gradients", precision, n, n, dev, uniform_core)
+    u, g = _out(x), _out(x)
+    code = _lib.precision_code(precision, uniform_core)
+    ws, nb, _keep = _scratch("velocity_and_strength_gradients", code, n, n, dev)
     _lib.check(_lib.load().vpm_velocity_and_strength_gradients(
-        _ptr(x), _ptr(a), _ptr(s), n, _ptr(u), _ptr(g),
-        _lib.precision_code(precision, uniform_core),
-        _ptr(ws), ws.numel(), _stream(dev)))
+        x.data_ptr(), a.data_ptr(), s.data_ptr(), n, u.data_ptr(), g.data_ptr(), code, ws, nb,
+        _stream(dev)))
     return u, g
 
 
@@ -183,12 +206,12 @@ def strength_gradients_pse(positions, strengths, radii, viscosities,
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     v = _check_scalar("viscosities", viscosities, n)
     _same_device(x, v)
-    out = torch.empty((n, 3), dtype=_F64, device=dev)
-    ws, nb = _workspace("strength_gradients_pse", precision, n, n, dev, uniform_core)
+    out = _out(x)
+    code = _lib.precision_code(precision, uniform_core)
+    ws, nb, _keep = _scratch("strength_gradients_pse", code, n, n, dev)
     _lib.check(_lib.load().vpm_strength_gradients_pse(
-        _ptr(x), _ptr(a), _ptr(s), _ptr(v), n, _ptr(out),
-        _lib.precision_code(precision, uniform_core),
-        _ptr(ws), ws.numel(), _stream(dev)))
+        x.data_ptr(), a.data_ptr(), s.data_ptr(), v.data_ptr(), n, out.data_ptr(), code, ws, nb,
+        _stream(dev)))
     return out
 
 
@@ -197,11 +220,12 @@ def _probe(fn_name, op, targets, positions, strengths, radii, precision):
     t = _check_vec("targets", targets)
     _same_device(x, t)
     m = t.shape[0]
-    out = torch.empty((m, 3), dtype=_F64, device=dev)
-    ws, nb = _workspace(op, precision, m, n, dev)
+    out = _out(t)
+    code = _lib.precision_code(precision)
+    ws, nb, _keep = _scratch(op, code, m, n, dev)
     fn = getattr(_lib.load(), fn_name)
-    _lib.check(fn(_ptr(t), m, _ptr(x), _ptr(a), _ptr(s), n, _ptr(out),
-                  _lib.precision_code(precision), _ptr(ws), ws.numel(), _stream(dev)))
+    _lib.check(fn(t.data_ptr(), m, x.data_ptr(), a.data_ptr(), s.data_ptr(), n, out.data_ptr(),
+                  code, ws, nb, _stream(dev)))
     return out
 
 
