@@ -179,16 +179,15 @@ struct Sweep {
     DevInfo d;
     int rc = device_info(&d);
     if (rc) return rc;
-    int occ = 0;
     {
+      // once per device: the shared-memory attribute, and the query that loads the kernel, so that
+      // a stream capture after the plan only launches
       int dev = 0;
       cudaGetDevice(&dev);
       const auto key = std::make_pair(static_cast<const void*>(kernel()), dev);
       std::lock_guard<std::mutex> lk(g_mu);
-      auto it = g_occ.find(key);
-      if (it != g_occ.end()) {
-        occ = it->second;
-      } else {
+      if (g_occ.find(key) == g_occ.end()) {
+        int occ = 0;
         if (kSmem > 48 * 1024) {
           cudaError_t e = cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                int(kSmem));
@@ -200,7 +199,6 @@ struct Sweep {
         g_occ[key] = occ;
       }
     }
-    if (occ < 1) occ = 1;
     const int64_t per_block = int64_t(C::THREADS) * R;
     p->tblocks = (m + per_block - 1) / per_block;
     p->smem = kSmem;
@@ -210,7 +208,18 @@ struct Sweep {
     p->splits = 1;
     p->chunk = n;
     if (n <= 0 || m <= 0) return VPM_OK;
-    const double slots = double(d.sms) * occ;
+    // Time of s splits, in units of one source for one block's targets on a busy SM: the blocks of
+    // the busiest SM, two at a time at least (fewer do not keep its pipes full) and half a block
+    // for the uneven end, each with a start and an end of about 24 sources, and the finalize's
+    // pass over the sets at 5 TB/s.  Against the fill of whole waves of resident blocks, which
+    // ignores that an SM with fewer blocks runs each faster (us): FP32c fused 623 -> 571 and
+    // velocity 332 -> 306 at 20000, 862 -> 799 and 459 -> 429 at 24000, adjoint 2195 -> 2045;
+    // FP64 test filter 47 -> 37 at 3000, energy gradient 43 -> 29 at 1500, probe vorticity of
+    // 10000 targets and sources 170 -> 158.
+    constexpr bool kFP32 = LaneTraits<T>::kLanes == 2;
+    constexpr double kOps = (kFP32 ? 13.0 : 18.0) + 3.0 * NV;  // of a pair, about
+    const double unit = double(C::THREADS) * R * kOps / (kFP32 ? 95.0 : 50.0);  // SM clocks
+    const double set = double(m) * NV * 16.0 / 5e12 * 1.9e9 / unit;
     double best = -1.0;
     for (int s = 1; s <= kMaxSplits; ++s) {
       int64_t chunk = (n + s - 1) / s;
@@ -219,11 +228,11 @@ struct Sweep {
       const int64_t se = (n + chunk - 1) / chunk;
       if (se != s) continue;
       if (size_t(se) * NV * size_t(m) * sizeof(double) > max_partial_bytes) break;
-      const double waves = double(p->tblocks) * se / slots;
-      const double eff = waves / std::ceil(waves);
-      const double score = eff * (1.0 - 0.003 * (se - 1));
-      if (score > best + 1e-12) {
-        best = score;
+      const double blocks = std::ceil(double(p->tblocks) * double(se) / d.sms);
+      const double cost = (double(chunk) + 24.0) * ((blocks > 2.0 ? blocks : 2.0) + 0.5) +
+                          double(se) * set;
+      if (best < 0.0 || cost < best) {
+        best = cost;
         p->splits = int(se);
         p->chunk = chunk;
       }
