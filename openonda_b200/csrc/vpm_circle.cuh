@@ -198,8 +198,7 @@ rot64_lists_kernel(const Sweep64Args a) {
       for (int v = 0; v < NV; ++v) jv[v] = 0.0;
 #pragma unroll Op::kUnroll
       for (int st = 0; st < 32; ++st) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) Op::pair2(tg[r], acc[r], jv, cur);
+        Op::pairs(tg, acc, jv, cur);
         Op::shuffle(cur, src_lane);
 #pragma unroll
         for (int v = 0; v < NJ; ++v)

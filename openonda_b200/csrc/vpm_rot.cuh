@@ -237,6 +237,30 @@ struct RotStd {
   __device__ __forceinline__ static constexpr bool long_fold(int) { return false; }
 };
 
+// A pair's distance and core: what its root needs.  The both-sides operators are split into this
+// head, the root y = x^(-1/2) and a tail that adds the pair's terms for both particles, so that
+// the FP64 kernels can form the heads and roots of all of a lane's targets before the first tail.
+template <class W>
+struct PairHead {
+  W rx, ry, rz, sg, s2, r2, x;  // r2: where the operator needs it apart from x
+};
+template <bool UC, class W, class TgtW, class SrcW>
+__device__ __forceinline__ PairHead<W> pair_head(const TgtW& t, const SrcW& s) {
+  PairHead<W> h;
+  h.rx = t.x - s.x;
+  h.ry = t.y - s.y;
+  h.rz = t.z - s.z;
+  if constexpr (UC) {
+    h.sg = t.sc;
+    h.s2 = t.s2c;
+  } else {
+    h.sg = fma(s.s, splat<W>(0.5), t.hs);
+    h.s2 = h.sg * h.sg;
+  }
+  h.x = fma(h.rx, h.rx, fma(h.ry, h.ry, fma(h.rz, h.rz, h.s2)));
+  return h;
+}
+
 // Fused velocity + stretching, both sides of the pair (FP32x2 lanes).  Built for 3 and for 2
 // resident CTAs per SM (MINB); the planner takes the one whose launches fill the waves better.
 template <bool REFINE, bool UC, int MINB = VPM_ROT_MINB, int P = VPM_ROT_P>
@@ -257,14 +281,20 @@ struct OpVelStretchBoth : RotStd<OpVelStretch<float2, REFINE, UC>, UC> {
   // one unordered pair for both particles, in any lane type (float2 here; double in the FP64
   // operator below)
   template <class W>
+  __device__ __forceinline__ static PairHead<W> head(const Tgt<W>& t, const Src<W>& s) {
+    return pair_head<UC, W>(t, s);
+  }
+  template <class W>
   __device__ __forceinline__ static void pair2(const Tgt<W>& t, W* acc, W* jv,
                                                const Src<W>& s) {
+    const PairHead<W> h = head(t, s);
+    tail(t, acc, jv, s, h, rsqrt_lane<REFINE>(h.x));
+  }
+  template <class W>
+  __device__ __forceinline__ static void tail(const Tgt<W>& t, W* acc, W* jv, const Src<W>& s,
+                                              const PairHead<W>& hd, W y) {
     using V = W;
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    V sg, s2;
-    pair_core<UC>(t, s, sg, s2);
-    const V x = fma(rx, rx, fma(ry, ry, fma(rz, rz, s2)));
-    const V y = rsqrt_lane<REFINE>(x);
+    const V rx = hd.rx, ry = hd.ry, rz = hd.rz, s2 = hd.s2, x = hd.x;
     const V y2 = y * y;
     V g, f;
     if constexpr (UC) {
@@ -322,14 +352,20 @@ struct OpVelBoth : RotStd<OpVel<float2, REFINE, UC>, UC> {
   static constexpr int kSymFrom = NV;
   static constexpr int kJBufs = 2;
   template <class W>
+  __device__ __forceinline__ static PairHead<W> head(const Tgt<W>& t, const Src<W>& s) {
+    return pair_head<UC, W>(t, s);
+  }
+  template <class W>
   __device__ __forceinline__ static void pair2(const Tgt<W>& t, W* acc, W* jv,
                                                const Src<W>& s) {
+    const PairHead<W> h = head(t, s);
+    tail(t, acc, jv, s, h, rsqrt_lane<REFINE>(h.x));
+  }
+  template <class W>
+  __device__ __forceinline__ static void tail(const Tgt<W>& t, W* acc, W* jv, const Src<W>& s,
+                                              const PairHead<W>& hd, W y) {
     using V = W;
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    V sg, s2;
-    pair_core<UC>(t, s, sg, s2);
-    const V x = fma(rx, rx, fma(ry, ry, fma(rz, rz, s2)));
-    const V y = rsqrt_lane<REFINE>(x);
+    const V rx = hd.rx, ry = hd.ry, rz = hd.rz, s2 = hd.s2, x = hd.x;
     const V y2 = y * y;
     V g;
     if constexpr (UC) {
@@ -361,14 +397,20 @@ struct OpStretchBoth {
   static constexpr int kSymFrom = NV;
   static constexpr bool kCustomDiag = false;
   template <class W>
+  __device__ __forceinline__ static PairHead<W> head(const Tgt<W>& t, const Src<W>& s) {
+    return pair_head<UC, W>(t, s);
+  }
+  template <class W>
   __device__ __forceinline__ static void pair2(const Tgt<W>& t, W* acc, W* jv,
                                                const Src<W>& s) {
+    const PairHead<W> h = head(t, s);
+    tail(t, acc, jv, s, h, rsqrt_lane<false>(h.x));
+  }
+  template <class W>
+  __device__ __forceinline__ static void tail(const Tgt<W>& t, W* acc, W* jv, const Src<W>& s,
+                                              const PairHead<W>& hd, W y) {
     using V = W;
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    V sg, s2;
-    pair_core<UC>(t, s, sg, s2);
-    const V x = fma(rx, rx, fma(ry, ry, fma(rz, rz, s2)));
-    const V y = rsqrt_lane<false>(x);
+    const V rx = hd.rx, ry = hd.ry, rz = hd.rz, s2 = hd.s2, x = hd.x;
     const V y2 = y * y;
     const V y5 = (y2 * y2) * y;
     const V t1 = fma(splat<V>(1.5), s2, x);
@@ -410,14 +452,20 @@ struct OpPseBoth : RotStd<OpPse<float2, REFINE, UC>, UC> {
   static constexpr int kSymFrom = NV;
   static constexpr int kJBufs = 2;
   template <class W>
+  __device__ __forceinline__ static PairHead<W> head(const Tgt<W>& t, const Src<W>& s) {
+    return pair_head<UC, W>(t, s);
+  }
+  template <class W>
   __device__ __forceinline__ static void pair2(const Tgt<W>& t, W* acc, W* jv,
                                                const Src<W>& s) {
+    const PairHead<W> h = head(t, s);
+    tail(t, acc, jv, s, h, rsqrt_lane<REFINE>(h.x));
+  }
+  template <class W>
+  __device__ __forceinline__ static void tail(const Tgt<W>& t, W* acc, W* jv, const Src<W>& s,
+                                              const PairHead<W>& hd, W y) {
     using V = W;
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    V sg, s2;
-    pair_core<UC>(t, s, sg, s2);
-    const V x = fma(rx, rx, fma(ry, ry, fma(rz, rz, s2)));
-    const V y = rsqrt_lane<REFINE>(x);
+    const V rx = hd.rx, ry = hd.ry, rz = hd.rz, sg = hd.sg;
     const V z = sg * y;  // <= 1
     const V z2 = z * z;
     const V z4 = z2 * z2;
@@ -473,15 +521,27 @@ struct OpLesStepBoth : RotStd<OpLesStep<float2, REFINE, UC>, UC> {
   __device__ __forceinline__ static constexpr bool carried(int v) { return v < kSymFrom; }
   static constexpr bool kCustomDiag = true;  // the FP64 kernel calls diag<double>
   template <class W>
+  __device__ __forceinline__ static PairHead<W> head(const Tgt<W>& t, const Src<W>& s) {
+    PairHead<W> h;
+    h.rx = t.x - s.x;
+    h.ry = t.y - s.y;
+    h.rz = t.z - s.z;
+    pair_core<UC>(t, s, h.sg, h.s2);
+    h.r2 = fma(h.rx, h.rx, fma(h.ry, h.ry, h.rz * h.rz));
+    h.x = h.r2 + h.s2;
+    return h;
+  }
+  template <class W>
   __device__ __forceinline__ static void pair2(const Tgt<W>& t, W* acc, W* jv,
                                                const Src<W>& s) {
+    const PairHead<W> h = head(t, s);
+    tail(t, acc, jv, s, h, rsqrt_lane<REFINE>(h.x));
+  }
+  template <class W>
+  __device__ __forceinline__ static void tail(const Tgt<W>& t, W* acc, W* jv, const Src<W>& s,
+                                              const PairHead<W>& hd, W y) {
     using V = W;
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    V sg, s2;
-    pair_core<UC>(t, s, sg, s2);
-    const V r2 = fma(rx, rx, fma(ry, ry, rz * rz));
-    const V x = r2 + s2;
-    const V y = rsqrt_lane<REFINE>(x);
+    const V rx = hd.rx, ry = hd.ry, rz = hd.rz, s2 = hd.s2, r2 = hd.r2, x = hd.x;
     const V y2 = y * y;
     const V y3 = y2 * y;
     const V y5 = y3 * y2;
@@ -651,14 +711,20 @@ struct OpRhsVjpBoth {
 
   // in any lane type (float2 here; double in the FP64 operator below)
   template <class W>
+  __device__ __forceinline__ static PairHead<W> head(const TgtGM<W>& t, const SrcG<W>& s) {
+    return pair_head<false, W>(t, s);
+  }
+  template <class W>
   __device__ __forceinline__ static void pair2(const TgtGM<W>& t, W* acc, W* jv,
                                                const SrcG<W>& s) {
+    const PairHead<W> h = head(t, s);
+    tail(t, acc, jv, s, h, rsqrt_lane<REFINE>(h.x));
+  }
+  template <class W>
+  __device__ __forceinline__ static void tail(const TgtGM<W>& t, W* acc, W* jv,
+                                              const SrcG<W>& s, const PairHead<W>& hd, W y) {
     using V = W;
-    const V rx = t.x - s.x, ry = t.y - s.y, rz = t.z - s.z;
-    const V sg = fma(s.s, splat<V>(0.5), t.hs);
-    const V s2 = sg * sg;
-    const V x = fma(rx, rx, fma(ry, ry, fma(rz, rz, s2)));
-    const V y = rsqrt_lane<REFINE>(x);
+    const V rx = hd.rx, ry = hd.ry, rz = hd.rz, sg = hd.sg, s2 = hd.s2, x = hd.x;
     const V y2 = y * y;
     const V y5 = (y2 * y2) * y;
     const V y7 = y5 * y2;
@@ -1025,15 +1091,19 @@ rot_sweep_kernel(const RotArgs a) {
 #ifndef VPM_ROT64_MINB
 #define VPM_ROT64_MINB 2
 #endif
-// Tuning of the FP64 builds, Gpairs/s at 131072 particles (fused / velocity / PSE): R = 4, two
-// CTAs per SM and four steps unrolled 459 / 766 / 967; two steps unrolled and (velocity, PSE)
-// three CTAs per SM 456 / 742 / 945; R = 2 and three CTAs 427 / 695 / 842; R = 2 and four CTAs
-// 410 / 675 / 827; R = 6 426 (one CTA) / 765 / 927.  Two warps per scheduler with four targets'
-// chains each hide more of the FP64 latency than more warps with fewer, whose shuffles double.
+// Tuning of the FP64 builds, Gpairs/s at 131072 particles (fused / velocity / PSE): R = 4 with two
+// CTAs per SM 456 / 766 / 967; R = 2 and three CTAs 427 / 695 / 842; R = 2 and four CTAs 410 / 675
+// / 827; R = 6 426 (one CTA) / 765 / 927.  The kernels wait for the latency of dependent FP64
+// operations with the pipe 72 % active; two warps per scheduler with four targets' chains each
+// hide more of it than more warps with fewer, whose shuffles double.  With the heads and roots of
+// a lane's targets formed first (`pairs`), one step unrolled and the prefetch per operator below,
+// at 65536 (fused / velocity / PSE / stretching / LES) 463 / 764 / 962 / 604 / 261 -> 473 / 805 /
+// 964 / 616 / 267.
 
 // Both32: the FP32 both-sides operator whose pair2 (a template in the lane type) gives the
 // pair terms; OneSided64: the one-sided FP64 operator of the diagonal tiles.
-template <class Both32, class OneSided64, bool UC, int UNROLL = 4, int P = VPM_ROT64_P>
+template <class Both32, class OneSided64, bool UC, int UNROLL, bool PREFETCH,
+          int P = VPM_ROT64_P>
 struct OpBoth64 {
   using V = double;
   using Record = Rec<double>;
@@ -1045,7 +1115,8 @@ struct OpBoth64 {
   static constexpr int kP = P;  // rot_tile: 64 kP warps = 32 R warps
   static constexpr int kMinBlocks = VPM_ROT64_MINB;
   static constexpr int kUnroll = UNROLL;  // of a batch's 32 steps
-  static constexpr bool kPrefetch = true;  // the next batch's source loads under this one's sums
+  // whether the next batch's source is loaded under this one's sums (14 to 16 registers)
+  static constexpr bool kPrefetch = PREFETCH;
   // values from kSymFrom on are taken once per unordered pair on the target side only
   static constexpr int kSymFrom = Both32::kSymFrom;
   static constexpr bool kUniformCore = UC;
@@ -1080,9 +1151,18 @@ struct OpBoth64 {
     t.s2c = s2;
     t.s4c = s2 * s2;
   }
-  __device__ __forceinline__ static void pair2(const TgtT& t, double* acc, double* jv,
-                                               const SrcT& s) {
-    Both32::pair2(t, acc, jv, s);
+  // the source against a lane's R targets: heads, roots, then the tails
+  template <int R>
+  __device__ __forceinline__ static void pairs(const TgtT (&t)[R], double (&acc)[R][NV],
+                                               double* jv, const SrcT& s) {
+    PairHead<double> h[R];
+    double y[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) h[r] = Both32::head(t[r], s);
+#pragma unroll
+    for (int r = 0; r < R; ++r) y[r] = rsqrt_fp64(h[r].x);
+#pragma unroll
+    for (int r = 0; r < R; ++r) Both32::tail(t[r], acc[r], jv, s, h[r], y[r]);
   }
   __device__ __forceinline__ static void diag(const TgtT& t, double* acc, const SrcT& s,
                                               const int64_t*, int64_t) {
@@ -1094,17 +1174,18 @@ struct OpBoth64 {
 };
 template <bool UC>
 using OpVelStretchBoth64 =
-    OpBoth64<OpVelStretchBoth<false, UC>, OpVelStretch<double, false, UC>, UC>;
+    OpBoth64<OpVelStretchBoth<false, UC>, OpVelStretch<double, false, UC>, UC, 1, true>;
 template <bool UC>
-using OpVelBoth64 = OpBoth64<OpVelBoth<false, UC>, OpVel<double, false, UC>, UC>;
+using OpVelBoth64 = OpBoth64<OpVelBoth<false, UC>, OpVel<double, false, UC>, UC, 1, true>;
 template <bool UC>
-using OpPseBoth64 = OpBoth64<OpPseBoth<false, UC>, OpPse<double, false, UC>, UC>;
+using OpPseBoth64 = OpBoth64<OpPseBoth<false, UC>, OpPse<double, false, UC>, UC, 2, false>;
 // the LES step's 13 sums: two FP64 targets per lane (256-particle tiles)
 template <bool UC>
 using OpLesStepBoth64 =
-    OpBoth64<OpLesStepBoth<false, UC>, OpLesStep<double, false, UC>, UC, 2, 1>;
+    OpBoth64<OpLesStepBoth<false, UC>, OpLesStep<double, false, UC>, UC, 1, false, 1>;
 template <bool UC>
-using OpStretchBoth64 = OpBoth64<OpStretchBoth<UC>, OpStretch<double, false, UC>, UC>;
+using OpStretchBoth64 =
+    OpBoth64<OpStretchBoth<UC>, OpStretch<double, false, UC>, UC, 1, false>;
 
 // The adjoint of (u, S [+ P]) in FP64 (OpRhsVjpBoth's pair terms): 14 or 18 sums and 16 or 17
 // travelling values leave room for two targets per lane.
@@ -1154,9 +1235,18 @@ struct OpRhsVjpBoth64 {
     for (int q = 0; q < Both32::kLaneValues; ++q)
       *v[q] = __shfl_sync(0xffffffffu, *v[q], src_lane);
   }
-  __device__ __forceinline__ static void pair2(const TgtT& t, double* acc, double* jv,
-                                               const SrcT& s) {
-    Both32::pair2(t, acc, jv, s);
+  // the source against a lane's R targets: heads, roots, then the tails
+  template <int R>
+  __device__ __forceinline__ static void pairs(const TgtT (&t)[R], double (&acc)[R][NV],
+                                               double* jv, const SrcT& s) {
+    PairHead<double> h[R];
+    double y[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) h[r] = Both32::head(t[r], s);
+#pragma unroll
+    for (int r = 0; r < R; ++r) y[r] = rsqrt_fp64(h[r].x);
+#pragma unroll
+    for (int r = 0; r < R; ++r) Both32::tail(t[r], acc[r], jv, s, h[r], y[r]);
   }
   __device__ __forceinline__ static void diag(const TgtT& t, double* acc, const SrcT& s,
                                               const int64_t* ti, int64_t j) {
@@ -1215,12 +1305,12 @@ rot64_sweep_kernel(const RotArgs a) {
     for (int v = 0; v < NV; ++v) jv[v] = 0.0;
 #pragma unroll Op::kUnroll
     for (int st = 0; st < 32; ++st) {
+      if constexpr (DIAG) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if constexpr (DIAG)
+        for (int r = 0; r < R; ++r)
           Op::diag(tg[r], acc[r], cur, &ti[r], j0 + b * 32 + ((lane + st) & 31));
-        else
-          Op::pair2(tg[r], acc[r], jv, cur);
+      } else {
+        Op::pairs(tg, acc, jv, cur);
       }
       // the source and its sums one lane down; after 32 steps both are back in their lane
       Op::shuffle(cur, src_lane);
