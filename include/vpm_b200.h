@@ -162,16 +162,16 @@ int vpm_velocity_and_strength_gradients(const double* positions, const double* s
  * vpm_strength_gradients_pse, vpm_les_step_sums, vpm_rhs_vjp, and vpm_sweep_records over all
  * records) with n >= this value evaluate each unordered pair once for both particles
  * (deterministic tile-pair schedule).  While the partial sums of a triangle of tile pairs fit
- * 2 GB (up to 70000 to 400000 particles, by operator and precision) that is one launch beside the
- * diagonal tiles'; past it about n / (2 T m) launches for tiles of T = 512 or 768 particles and m
- * diagonal pairs per launch.  The diagonal tiles of the triangle, and of short launches, run on a
- * second stream of the library's, forked from and joined to the caller's stream by events inside
- * the call, so stream order and CUDA-graph capture see one call as before; that stream is created
- * by the first such call in a context (make it before any stream capture).  The FP64 self sums (those above, the stretching and
- * the adjoint among them) do so from a sixth of this value on, in one launch over a circle of
- * tiles; the stretching and the adjoint stay there while their partial sums fit 4 GB.  The scalar
- * diagnostics in FP64 take each unordered pair once at every size.  Sets the threshold and
- * returns the previous one (default 24576).  No counterpart in the reference. */
+ * 2 GB (FP32c: and n is at most 150000) that is one launch beside the diagonal tiles'; past it
+ * about n / (2 T m) launches for tiles of T = 512 or 768 particles and m diagonal pairs per
+ * launch.  The diagonal tiles of the triangle, and of short launches, run on a second stream of
+ * the library's, forked from and joined to the caller's stream by events inside the call, so
+ * stream order and CUDA-graph capture see one call as before; that stream is created by the first
+ * such call in a context (make it before any stream capture).  The FP64 self sums (those above,
+ * the stretching and the adjoint among them) do so from a sixth of this value on, in one launch
+ * over a circle of tiles; the stretching and the adjoint stay there while their partial sums fit
+ * 4 GB.  The scalar diagnostics in FP64 take each unordered pair once at every size.  Sets the
+ * threshold and returns the previous one (default 24576).  No counterpart in the reference. */
 int64_t vpm_set_symmetric_min_n(int64_t n);
 /* Kernel launches of one sweep of `op` (sweep and finalize, not the packing of the inputs)
  * for m targets and n sources under the current plan; -1 on error.  1: a small sum, whose one

@@ -971,8 +971,11 @@ __global__ void finalize_kegrad_kernel(const double* __restrict__ part, int spli
 
 // ---- both-sides sweep over a triangle of tile pairs (vpm_triangle.cuh, vpm_circle.cuh) --------
 // Its partial sums may take this much; past it the sweep is the many-launch one (vpm_rot.cuh),
-// whose accumulators do not grow with n^2.
+// whose accumulators do not grow with n^2.  In FP32c the many-launch sweep's waves are long enough
+// from about 150000 particles: velocity 1844 -> 1860 Gpairs/s with the triangle at 140000, 1876 ->
+// 1868 at 200000, 1896 -> 1873 at 330000, fused 963 -> 991 at 140000 and 991 -> 990 at 262144.
 constexpr size_t kMaxTriangleBytes = size_t(2) << 30;
+constexpr int64_t kMaxTriangleN32 = 150000;
 
 template <class Op>
 struct TriSweep {
@@ -1022,8 +1025,9 @@ struct TriSweep {
     int rc = device_info(&d);
     if (!rc) rc = prepare(&occ);
     if (!rc) rc = RotSweep<Op>::prepare_side();
-    if (rc || n >= (int64_t(1) << 30)) return rc;
+    if (rc || n >= (int64_t(1) << 30) || (!Op::kFP64 && n > kMaxTriangleN32)) return rc;
     const TriLists l(n, kTile, kUnit);
+    if (size_t(l.nt / 2) * NV * size_t(n) * sizeof(double) > kMaxTriangleBytes) return VPM_OK;
     const Shares shares = Shares::make(l.total(), int64_t(d.sms) * occ);
     const int tsets = target_sets(l, shares);
     const int64_t sets =
@@ -1125,6 +1129,8 @@ struct CircleSweep {
     if (!rc) rc = prepare(&occ);
     if (rc) return rc;
     const CircleLists l(n, kTile);
+    // (the source sets alone: no count of the target sets at sizes that are far past the budget)
+    if (size_t(l.half) * NV * size_t(n) * sizeof(double) > max_partial_bytes) return VPM_OK;
     p->shares = Shares::make(l.total(), int64_t(d.sms) * occ);
     const int64_t sets = target_sets(l, p->shares) + l.half;
     if (size_t(sets) * NV * size_t(n) * sizeof(double) > max_partial_bytes) return VPM_OK;
