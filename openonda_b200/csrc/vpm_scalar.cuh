@@ -16,8 +16,10 @@
 // (two-sum), so the total is rounded once or twice instead of some twenty times.
 //
 // Bound: the FP64 pipe (28 / 21 / 28 operations per unordered pair).  Measured against the
-// one-sided sweeps (us, kinetic energy / enstrophy / helicity): 2311 / 1819 / 2173 -> 1099 / 876
-// / 1073 at 32768 particles, 69 / 59 / 67 -> 26 / 23 / 25 at 4096.
+// one-sided sweeps (us, kinetic energy / enstrophy / helicity): 2311 / 1819 / 2173 -> 1069 / 779
+// / 1022 at 32768 particles, 69 / 59 / 67 -> 25 / 20 / 25 at 4096.  Two targets per thread and
+// eight sources unrolled; four sources 1078 / 815 / 1046, two 1100 / 877 / 1070, one 1147 / 941 /
+// 1099, four targets 1139 / 877 / 1109 at 32768.
 #pragma once
 
 #include "vpm_sweep.cuh"
@@ -184,7 +186,7 @@ scalar_pairs_kernel(const ScalarArgs a) {
           for (int r = 0; r < R; ++r) acc[r] *= 0.5;
         }
       } else {
-#pragma unroll 2
+#pragma unroll 8
         for (int j = 0; j < cnt; ++j) {
           const Src<double> src = load_src<double>(ring[s][j]);
 #pragma unroll
