@@ -117,10 +117,18 @@ __device__ __forceinline__ void pair_core(const Tgt<V>& t, const Src<V>& s, V& s
 template <class V>
 constexpr int kProbeR = LaneTraits<V>::kLanes == 1 ? 2 : 0;
 
+// Sources unrolled in the one-sided FP64 velocity, fused and PSE sums (one target per thread):
+// with the branch-free root four interleave better than two (fused 363 -> 364, PSE 603 -> 611,
+// velocity 530 -> 568 Gpairs/s at 65536 against the branching root with two; with two 356 / 589 /
+// 574).  The stretching takes two targets instead (384 -> 391; 380 with four sources).
+template <class V>
+constexpr int kSelfUnroll = LaneTraits<V>::kLanes == 1 ? 4 : 2;
+
 // Record/lane plumbing shared by the operators on the standard 64-byte record.
 template <class V>
 struct PairOpBase {
   static constexpr bool kGuarded = false;  // pairs within r^2 <= kRefEps are skipped (see OpVelAt)
+  static constexpr int kSrcUnroll = 2;     // sources unrolled in the one-sided sweep
   static constexpr int kR = 0;  // targets per thread: 0 = the precision's default
   // FP32 sources per FP64 carry fold of the one-sided sweep: 0 = the sweep's default (32)
   static constexpr int kWindow = 0;
@@ -134,6 +142,7 @@ struct PairOpBase {
 // ---- self-induced velocity: U += g (r x a_j) ------------------------------------------
 template <class V, bool REFINE, bool UC = false>
 struct OpVel : PairOpBase<V> {
+  static constexpr int kSrcUnroll = kSelfUnroll<V>;
   static constexpr int NV = 3;
   __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
                                               const int64_t*, int64_t) {
@@ -287,6 +296,7 @@ struct OpTestFilter {
   static constexpr int NV = 5;
   static constexpr int kR = kProbeR<V>;
   static constexpr int kWindow = 0;
+  static constexpr int kSrcUnroll = 2;
   static constexpr bool kGuarded = true;
   static constexpr int kGuardGroup = 4;
   using Record = RecF<V>;
@@ -321,6 +331,7 @@ struct OpTestFilter {
 // ---- stretching (transpose scheme): A += g (a_j - a_i),  B += f (r . (d x a_i)) r -------
 template <class V, bool REFINE, bool UC = false>
 struct OpStretch : PairOpBase<V> {
+  static constexpr int kR = LaneTraits<V>::kLanes == 1 ? 2 : 0;
   static constexpr int NV = 6;
   static constexpr int kWindow = VPM_STRETCH_WINDOW;
   __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
@@ -355,6 +366,7 @@ struct OpStretch : PairOpBase<V> {
 #endif
 template <class V, bool REFINE, bool UC = false>
 struct OpVelStretch : PairOpBase<V> {
+  static constexpr int kSrcUnroll = kSelfUnroll<V>;
   static constexpr int NV = 9;
   static constexpr int kWindow = VPM_STRETCH_WINDOW;
   __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
@@ -457,6 +469,7 @@ struct OpLesStep : PairOpBase<V> {
 // ---- PSE diffusion: P += s^7 y^9 (a_j - a_i)  (nu_i applied in finalize) -----------------
 template <class V, bool REFINE, bool UC = false>
 struct OpPse : PairOpBase<V> {
+  static constexpr int kSrcUnroll = kSelfUnroll<V>;
   static constexpr int NV = 3;
   __device__ __forceinline__ static void pair(const Tgt<V>& t, V* acc, const Src<V>& s,
                                               const int64_t*, int64_t) {

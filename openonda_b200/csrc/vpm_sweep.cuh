@@ -43,10 +43,6 @@ struct SweepArgs {
 #ifndef VPM_SMEM_CARRY
 #define VPM_SMEM_CARRY 0
 #endif
-#ifndef VPM_SRC_UNROLL
-#define VPM_SRC_UNROLL 2
-#endif
-constexpr int kSrcUnroll = VPM_SRC_UNROLL;
 
 // Dynamic shared memory of one block: the source-tile ring, then (FP32 with shared-memory
 // carries) the FP64 carries laid out [value][target][thread] for conflict-free access.
@@ -174,7 +170,7 @@ sweep_kernel(const SweepArgs<typename Op::Record> a) {
             }
           }
         }
-#pragma unroll kSrcUnroll
+#pragma unroll Op::kSrcUnroll
         for (; j < e; ++j) {
           const typename Op::SrcT src = Op::load(tile[j]);
 #pragma unroll
