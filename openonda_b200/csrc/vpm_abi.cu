@@ -86,9 +86,7 @@ constexpr int kMaxSplits = VPM_MAX_SPLITS;
 // adjoint, 85 / 26 / 26 us for the FP64 and 42 / 22 / 24 us for the FP32c LES step sums.
 template <class T>
 constexpr int64_t kMinChunk = LaneTraits<T>::kLanes == 1 ? 32 : 64;
-// The scalar sums' finalize is one block that walks all splits: at 4096 particles and chunks of
-// 64 the FP32c kinetic energy took 74 us, of 256 45 us.
-constexpr int64_t kMinChunkScalar = 256;
+constexpr int64_t kMinChunkScalar = 256;  // of the scalar sums (Sweep::plan)
 constexpr size_t kMaxPartialBytes = size_t(4) << 30;
 
 struct Plan {
@@ -174,11 +172,13 @@ struct Sweep {
     return reinterpret_cast<void*>(&sweep_kernel<Op, T, R, C::THREADS, TILE, C::STAGES, C::MINB>);
   }
 
+  // scalar: the sum's finalize is the one block of finalize_dot_kernel
   static int plan(int64_t m, int64_t n, Plan* p, size_t max_partial_bytes = kMaxPartialBytes,
-                  int64_t min_chunk = kMinChunk<T>) {
+                  bool scalar = false) {
     DevInfo d;
     int rc = device_info(&d);
     if (rc) return rc;
+    int occ = 0;
     {
       // once per device: the shared-memory attribute, and the query that loads the kernel, so that
       // a stream capture after the plan only launches
@@ -186,8 +186,10 @@ struct Sweep {
       cudaGetDevice(&dev);
       const auto key = std::make_pair(static_cast<const void*>(kernel()), dev);
       std::lock_guard<std::mutex> lk(g_mu);
-      if (g_occ.find(key) == g_occ.end()) {
-        int occ = 0;
+      auto it = g_occ.find(key);
+      if (it != g_occ.end()) {
+        occ = it->second;
+      } else {
         if (kSmem > 48 * 1024) {
           cudaError_t e = cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                int(kSmem));
@@ -199,6 +201,7 @@ struct Sweep {
         g_occ[key] = occ;
       }
     }
+    if (occ < 1) occ = 1;
     const int64_t per_block = int64_t(C::THREADS) * R;
     p->tblocks = (m + per_block - 1) / per_block;
     p->smem = kSmem;
@@ -210,16 +213,20 @@ struct Sweep {
     if (n <= 0 || m <= 0) return VPM_OK;
     // Time of s splits, in units of one source for one block's targets on a busy SM: the blocks of
     // the busiest SM, two at a time at least (fewer do not keep its pipes full) and half a block
-    // for the uneven end, each with a start and an end of about 24 sources, and the finalize's
+    // for the uneven end, each with a start and an end of about 40 sources, and the finalize's
     // pass over the sets at 5 TB/s.  Against the fill of whole waves of resident blocks, which
     // ignores that an SM with fewer blocks runs each faster (us): FP32c fused 623 -> 571 and
     // velocity 332 -> 306 at 20000, 862 -> 799 and 459 -> 429 at 24000, adjoint 2195 -> 2045;
-    // FP64 test filter 47 -> 37 at 3000, energy gradient 43 -> 29 at 1500, probe vorticity of
-    // 10000 targets and sources 170 -> 158.
+    // probe vorticity of 10000 targets and sources in FP64 170 -> 158.  (Of 24, 40 and 12 sources,
+    // 40 left no sum slower than the waves at 15 sizes from 4500 to 24400.)
+    //
+    // The scalar sums keep the waves and long splits: their finalize is one block that walks all
+    // splits (FP32c kinetic energy 417 against 549 us at 20000, 45 against 74 at 4096).
     constexpr bool kFP32 = LaneTraits<T>::kLanes == 2;
     constexpr double kOps = (kFP32 ? 13.0 : 18.0) + 3.0 * NV;  // of a pair, about
     const double unit = double(C::THREADS) * R * kOps / (kFP32 ? 95.0 : 50.0);  // SM clocks
     const double set = double(m) * NV * 16.0 / 5e12 * 1.9e9 / unit;
+    const int64_t min_chunk = scalar ? kMinChunkScalar : kMinChunk<T>;
     double best = -1.0;
     for (int s = 1; s <= kMaxSplits; ++s) {
       int64_t chunk = (n + s - 1) / s;
@@ -228,10 +235,16 @@ struct Sweep {
       const int64_t se = (n + chunk - 1) / chunk;
       if (se != s) continue;
       if (size_t(se) * NV * size_t(m) * sizeof(double) > max_partial_bytes) break;
-      const double blocks = std::ceil(double(p->tblocks) * double(se) / d.sms);
-      const double cost = (double(chunk) + 24.0) * ((blocks > 2.0 ? blocks : 2.0) + 0.5) +
-                          double(se) * set;
-      if (best < 0.0 || cost < best) {
+      const double total = double(p->tblocks) * double(se);
+      double cost;
+      if (scalar) {
+        const double waves = total / (double(d.sms) * occ);
+        cost = std::ceil(waves) / waves / (1.0 - 0.003 * double(se - 1));
+      } else {
+        const double blocks = std::ceil(total / d.sms);
+        cost = (double(chunk) + 40.0) * ((blocks > 2.0 ? blocks : 2.0) + 0.5) + double(se) * set;
+      }
+      if (best < 0.0 || cost < best - 1e-12) {
         best = cost;
         p->splits = int(se);
         p->chunk = chunk;
@@ -1346,7 +1359,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarHel>::plan(n, p);
       }
-      return Sweep<typename O::Vel, T>::plan(m, n, p, mpb, kMinChunkScalar);
+      return Sweep<typename O::Vel, T>::plan(m, n, p, mpb, true);
     case VPM_OP_INDUCED_VELOCITY_AT:
       return plan_vector<typename O::VelAt, T, FIN_VEL>(m, n, p, mpb);
     case VPM_OP_VORTICITY_FIELD_AT:
@@ -1370,12 +1383,12 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarKe>::plan(n, p);
       }
-      return Sweep<typename O::Ke, T>::plan(m, n, p, mpb, kMinChunkScalar);
+      return Sweep<typename O::Ke, T>::plan(m, n, p, mpb, true);
     case VPM_OP_TOTAL_ENSTROPHY:
       if constexpr (LaneTraits<T>::kLanes == 1) {
         if (m == n && n > 0) return ScalarSweep<ScalarEns>::plan(n, p);
       }
-      return Sweep<typename O::Ens, T>::plan(m, n, p, mpb, kMinChunkScalar);
+      return Sweep<typename O::Ens, T>::plan(m, n, p, mpb, true);
     case VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
         if (RotSweep<typename O::VelStretchBoth>::usable(m, n, mpb)) {
