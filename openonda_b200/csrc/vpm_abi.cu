@@ -390,14 +390,31 @@ struct SetsFinalize {
   }
 };
 
-template <class T, int KIND, int NV>
-__global__ void finalize_vec_kernel(const double* __restrict__ part, int splits, int64_t m,
-                                    const SetsFinalize<T, KIND, NV> fin) {
+// One thread per particle; the sum over few splits, or of many particles.
+template <int NV, class Finalize>
+__global__ void finalize_kernel(const double* __restrict__ part, int splits, int64_t m,
+                                const Finalize fin) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= m) return;
   double v[NV];
   sum_splits<NV>(part, splits, m, i, v);
   fin.write(v, i);
+}
+
+// part: [splits][NV][m]; fin.write(v, i) takes the sums of particle i.
+template <int NV, class Finalize>
+int finalize(const double* part, int splits, int64_t m, const Finalize& fin, cudaStream_t st) {
+  if (m <= 0) return VPM_OK;
+  if (splits >= kSetLanesMinSplits && m <= kSetLanesMaxTargets) {
+    finalize_sets_kernel<NV, NV, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
+        part, SplitSets{splits}, m, fin);
+  } else {
+    const int threads = 256;
+    finalize_kernel<NV>
+        <<<unsigned((m + threads - 1) / threads), threads, 0, st>>>(part, splits, m, fin);
+  }
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
 }
 
 // Pair shards across GPUs: rows[i][v] = the sum over the sets s, in order, of acc[s][v][i].
@@ -478,19 +495,8 @@ template <class T, int KIND, int NV>
 int finalize_vec(const double* part, int splits, int64_t m, const Rec<T>* tgt, double* out,
                  double* out2, cudaStream_t st, double* out3 = nullptr,
                  double* scalar = nullptr) {
-  if (m <= 0) return VPM_OK;
-  const SetsFinalize<T, KIND, NV> fin{tgt, out, out2, out3, scalar};
-  if (splits >= kSetLanesMinSplits && m <= kSetLanesMaxTargets) {
-    finalize_sets_kernel<NV, NV, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
-        part, SplitSets{splits}, m, fin);
-  } else {
-    const int threads = 256;
-    finalize_vec_kernel<T, KIND, NV>
-        <<<unsigned((m + threads - 1) / threads), threads, 0, st>>>(part, splits, m, fin);
-  }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "finalize launch");
-  return VPM_OK;
+  return finalize<NV>(part, splits, m, SetsFinalize<T, KIND, NV>{tgt, out, out2, out3, scalar},
+                      st);
 }
 
 __global__ void zero_kernel(double* p, int64_t count) {
@@ -943,44 +949,20 @@ struct SetsFinalizeVjp {
   }
 };
 
-template <class E, bool PSE>
-__global__ void finalize_vjp_kernel(const double* __restrict__ part, int splits, int64_t m,
-                                    const SetsFinalizeVjp<E, PSE> fin) {
-  constexpr int NV = SetsFinalizeVjp<E, PSE>::NV;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  double v[NV];
-  sum_splits<NV>(part, splits, m, i, v);
-  fin.write(v, i);
-}
-
-template <class E, bool PSE>
-void finalize_vjp(const double* part, int splits, int64_t m, const SetsFinalizeVjp<E, PSE>& fin,
-                  cudaStream_t st) {
-  constexpr int NV = SetsFinalizeVjp<E, PSE>::NV;
-  if (splits >= kSetLanesMinSplits && m <= kSetLanesMaxTargets)
-    finalize_sets_kernel<NV, NV, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
-        part, SplitSets{splits}, m, fin);
-  else
-    finalize_vjp_kernel<E, PSE><<<unsigned((m + 255) / 256), 256, 0, st>>>(part, splits, m, fin);
-}
-
-__global__ void finalize_kegrad_kernel(const double* __restrict__ part, int splits, int64_t m,
-                                       double* __restrict__ gx, double* __restrict__ ga,
-                                       double* __restrict__ gsig) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  double v[7];
-  sum_splits<7>(part, splits, m, i, v);
-  const double c = 2.0 / (16.0 * kPi);
-  gx[3 * i] = c * v[0];
-  gx[3 * i + 1] = c * v[1];
-  gx[3 * i + 2] = c * v[2];
-  ga[3 * i] = c * v[3];
-  ga[3 * i + 1] = c * v[4];
-  ga[3 * i + 2] = c * v[5];
-  gsig[i] = 0.5 * c * v[6];
-}
+// Gradients of the kinetic energy (OpKeGrad's seven sums).
+struct SetsFinalizeKeGrad {
+  double *gx, *ga, *gs;
+  __device__ __forceinline__ void write(const double (&v)[7], int64_t i) const {
+    const double c = 2.0 / (16.0 * kPi);
+    gx[3 * i] = c * v[0];
+    gx[3 * i + 1] = c * v[1];
+    gx[3 * i + 2] = c * v[2];
+    ga[3 * i] = c * v[3];
+    ga[3 * i + 1] = c * v[4];
+    ga[3 * i + 2] = c * v[5];
+    gs[i] = 0.5 * c * v[6];
+  }
+};
 
 // ---- both-sides sweep over a triangle of tile pairs (vpm_triangle.cuh, vpm_circle.cuh) --------
 // Its partial sums may take this much; past it the sweep is the many-launch one (vpm_rot.cuh),
@@ -1822,21 +1804,18 @@ __global__ void pack_filter_kernel(const double* __restrict__ pos, const double*
 
 // w_hat (m,3) and the two filtered fields (m,3; third column 0), both with the zeta kernel's
 // 7.5/(4 pi) as in vpm_vorticity_field_at.
-template <class T>
-__global__ void finalize_filter_kernel(const double* __restrict__ part, int splits, int64_t m,
-                                       double* __restrict__ w_hat, double* __restrict__ f_hat) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  double v[5];
-  sum_splits<5>(part, splits, m, i, v);
-  const double c = 7.5 * kOneOver4Pi;
-  w_hat[3 * i] = v[0] * c;
-  w_hat[3 * i + 1] = v[1] * c;
-  w_hat[3 * i + 2] = v[2] * c;
-  f_hat[3 * i] = v[3] * c;
-  f_hat[3 * i + 1] = v[4] * c;
-  f_hat[3 * i + 2] = 0.0;
-}
+struct SetsFinalizeFilter {
+  double *w_hat, *f_hat;
+  __device__ __forceinline__ void write(const double (&v)[5], int64_t i) const {
+    const double c = 7.5 * kOneOver4Pi;
+    w_hat[3 * i] = v[0] * c;
+    w_hat[3 * i + 1] = v[1] * c;
+    w_hat[3 * i + 2] = v[2] * c;
+    f_hat[3 * i] = v[3] * c;
+    f_hat[3 * i + 1] = v[4] * c;
+    f_hat[3 * i + 2] = 0.0;
+  }
+};
 
 template <class T, bool REFINE>
 int run_filter(const Call& c) {
@@ -1863,9 +1842,7 @@ int run_filter(const Call& c) {
   if (e != cudaSuccess) return cuda_fail(e, "pack launch");
   rc = Sweep<Op, T>::launch(p, rec, c.n, 0, rec, c.n, part, c.st);
   if (rc) return rc;
-  finalize_filter_kernel<T><<<blocks, 256, 0, c.st>>>(part, p.splits, c.n, c.out, c.out2);
-  e = cudaGetLastError();
-  return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
+  return finalize<5>(part, p.splits, c.n, SetsFinalizeFilter{c.out, c.out2}, c.st);
 }
 
 // Decoded precision code: compute type, Newton-refined rsqrt, uniform cores.
@@ -1952,9 +1929,7 @@ int run_grad(const GradCall& c) {
     rc = pack<T>(c.pos, c.str, c.rad, nullptr, c.n, rec, c.st);
     if (!rc) rc = Sweep<typename O::KeGrad, T>::launch(p, rec, c.n, 0, rec, c.n, part, c.st);
     if (rc) return rc;
-    finalize_kegrad_kernel<<<blocks, 256, 0, c.st>>>(part, p.splits, c.n, c.ox, c.oa, c.os);
-    e = cudaGetLastError();
-    return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
+    return finalize<7>(part, p.splits, c.n, SetsFinalizeKeGrad{c.ox, c.oa, c.os}, c.st);
   }
   RecG<T>* rec = reinterpret_cast<RecG<T>*>(ws + L.src_off);
   pack_grad_kernel<T><<<blocks, 256, 0, c.st>>>(c.pos, c.str, c.rad, c.nu, c.gu, c.gs, c.n, rec);
@@ -1976,8 +1951,8 @@ int run_grad(const GradCall& c) {
     if (!p.pairs)
       rc = Sweep<typename O::RhsVjpPse, T>::launch(p, rec, c.n, 0, rec, c.n, part, c.st);
     if (rc) return rc;
-    finalize_vjp<T, true>(part, p.splits, c.n, SetsFinalizeVjp<T, true>{rec, c.ox, c.oa, c.os, c.onu},
-                        c.st);
+    rc = finalize<O::RhsVjpPse::NV>(part, p.splits, c.n,
+                             SetsFinalizeVjp<T, true>{rec, c.ox, c.oa, c.os, c.onu}, c.st);
   } else {
     rc = VPM_OK;
     if constexpr (LaneTraits<T>::kLanes == 2) {
@@ -1993,11 +1968,10 @@ int run_grad(const GradCall& c) {
     }
     if (!p.pairs) rc = Sweep<typename O::RhsVjp, T>::launch(p, rec, c.n, 0, rec, c.n, part, c.st);
     if (rc) return rc;
-    finalize_vjp<T, false>(part, p.splits, c.n, SetsFinalizeVjp<T, false>{rec, c.ox, c.oa, c.os, c.onu},
-                        c.st);
+    rc = finalize<O::RhsVjp::NV>(part, p.splits, c.n,
+                             SetsFinalizeVjp<T, false>{rec, c.ox, c.oa, c.os, c.onu}, c.st);
   }
-  e = cudaGetLastError();
-  return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
+  return rc;
 }
 
 int dispatch_grad(const GradCall& c, int precision) {

@@ -916,7 +916,7 @@ __device__ __forceinline__ void rot_batch(typename Op::Lane cur,
   static_assert(32 % SW == 0, "the source window divides the 32 steps of a batch");
   static_assert(32 % TW == 0 && TW % SW == 0, "target windows are whole source windows");
   constexpr int TWS = Op::kTgtWindowShort;
-  static_assert(TWS == 0 || (TW % TWS == 0 && TWS % SW == 0),
+  static_assert(TW % (TWS > 0 ? TWS : 1) == 0 && TWS % SW == 0,
                 "short target windows divide the target window and are whole source windows");
   constexpr int TWL = Op::kTgtWindowLong;
   static_assert(TWL == 0 || TWL % 32 == 0, "long target windows are whole batches");

@@ -49,7 +49,7 @@ rot_triangle_kernel(const TriArgs a) {
   constexpr int T = rot_tile<Op>();
   constexpr int NJ = Op::kSymFrom;
   static_assert(T % kTriUnit == 0, "tiles are whole units");
-  static_assert(Op::kTgtWindowLong == 0 || kTriUnit % Op::kTgtWindowLong == 0,
+  static_assert(kTriUnit % (Op::kTgtWindowLong > 0 ? Op::kTgtWindowLong : 1) == 0,
                 "units are whole target windows");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* car = reinterpret_cast<double*>(smem_raw);  // [NV][T]
