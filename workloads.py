@@ -185,7 +185,7 @@ def _pipe_peaks():
 
 # FP32 lane-ops and MUFU rsqrt per ordered pair of the fused velocity + stretching sum
 # (general cores): one-sided OpVelStretch 38 / 1, both-sides OpVelStretchBoth 26.5 / 0.5;
-# FP64 one-sided: 38 FP64 ops (DFMA pipe) and one rsqrt() per pair.
+# FP64 one-sided: 38 FP64 ops (DFMA pipe) and one root of five more per pair.
 _FUSED_OPS = {"one-sided": (38.0, 1.0), "both-sides": (26.5, 0.5)}
 
 
@@ -219,8 +219,10 @@ def config3(args):
             res[prec] = n * n / (best / 1e3) / 1e9
         path = ("both-sides" if kernels.sweep_launches("velocity_and_strength_gradients",
                                                         "fp32c", n, n) > 2 else "one-sided")
-        path64 = ("both-sides" if kernels.sweep_launches("velocity_and_strength_gradients",
-                                                          "fp64", n, n) > 2 else "one-sided")
+        # the one-sided FP64 sweep holds one target per thread, the both-sides forms four
+        path64 = ("both-sides" if kernels.plan_info("velocity_and_strength_gradients", "fp64", n,
+                                                    n)["targets_per_thread"] > 1
+                  else "one-sided")
         ops, rsq = _FUSED_OPS[path]
         ops64 = _FUSED_OPS[path64][0]  # the FP64 kernels execute the same pair terms
         r32 = res["fp32c"] * 1e9
