@@ -23,6 +23,8 @@
  *     with respect to the host; scalar results are written to a device double.
  *   - Return value: VPM_OK (0) or an error code; vpm_last_error() gives the message for
  *     the calling thread.  Inputs are never modified; nothing throws across the ABI.
+ *   - The pair sums read all of their input arrays before they write an output, so an output
+ *     may overlap the inputs (not the packed records of vpm_sweep_records).
  *   - Radii must be positive.  Results are deterministic for a given device and sizes.
  */
 #ifndef VPM_B200_H
@@ -175,7 +177,8 @@ int vpm_velocity_and_strength_gradients(const double* positions, const double* s
 int64_t vpm_set_symmetric_min_n(int64_t n);
 /* Kernel launches of one sweep of `op` (sweep and finalize, not the packing of the inputs)
  * for m targets and n sources under the current plan; -1 on error.  1: a small sum, whose one
- * launch also packs the caller's arrays (from packed records it takes sweep and finalize). */
+ * launch also packs the caller's arrays (from packed records it takes sweep and finalize, and
+ * so it does, after the pack, where an output overlaps an input). */
 int64_t vpm_sweep_launches(int op, int precision, int64_t m, int64_t n);
 
 /* The four pair sums of one dynamic-LES time step on the same state, in one sweep:

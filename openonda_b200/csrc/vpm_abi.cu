@@ -1508,6 +1508,27 @@ struct Call {
   const double* aux = nullptr;  // VPM_OP_LES_TEST_FILTER: the filtered fields (n,3)
 };
 
+// Whether an output of the call shares memory with one of its inputs.
+bool outputs_overlap_inputs(const Call& c) {
+  struct Range {
+    const double* p;
+    int64_t count;
+  };
+  const Range in[] = {{c.tgt, 3 * c.m}, {c.pos, 3 * c.n}, {c.str, 3 * c.n}, {c.rad, c.n},
+                      {c.nu, c.n}};
+  for (const double* out : {c.out, c.out2}) {
+    if (!out) continue;
+    const uintptr_t o = reinterpret_cast<uintptr_t>(out);
+    const uintptr_t o_end = o + size_t(3 * c.m) * sizeof(double);
+    for (const Range& r : in) {
+      if (!r.p) continue;
+      const uintptr_t i = reinterpret_cast<uintptr_t>(r.p);
+      if (o < i + size_t(r.count) * sizeof(double) && i < o_end) return true;
+    }
+  }
+  return false;
+}
+
 template <class T, bool REFINE, bool UC>
 int run(const Call& c) {
   using O = Ops<T, REFINE, UC>;
@@ -1539,7 +1560,9 @@ int run(const Call& c) {
   if (c.ws_bytes < L.total)
     return fail(VPM_ERR_WORKSPACE, "workspace has " + std::to_string(c.ws_bytes) +
                                        " bytes, needs " + std::to_string(L.total));
-  if (p.small && !c.records) {
+  // the one launch reads the caller's arrays until its last cluster is done, so outputs that
+  // overlap them take the packed route, which copies every input before it writes
+  if (p.small && !c.records && !outputs_overlap_inputs(c)) {
     const bool probe = is_probe(c.op);
     const SmallArgs a{probe ? c.tgt : c.pos, probe ? nullptr : c.str, c.nu,     c.pos,
                       c.str,                 c.rad,                   int(c.m), int(c.n),

@@ -12,6 +12,10 @@
 // The pair terms, the FP32 windows (whole multiples of Op::kWindow sources from a window's
 // start) and the FP64 carries are those of sweep_kernel, so results differ from it only by the
 // order of FP64 additions.  No scratch memory.
+//
+// There is no order between clusters: one writes its targets' outputs while another still reads
+// sources.  The outputs must therefore not overlap the inputs (the dispatch sends such calls
+// through packed records instead).
 #pragma once
 
 #include <cooperative_groups.h>
