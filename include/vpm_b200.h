@@ -56,6 +56,13 @@ enum vpm_precision { VPM_FP64 = 0, VPM_FP32C = 1, VPM_FP32C_REFINED = 2 };
  * word when a radius differs from radii[0] (results are then wrong).  Probe sums, the kinetic
  * energy and the adjoint ignore the flag.  No counterpart in the reference. */
 #define VPM_UNIFORM_CORE 0x100
+/* Flag OR-ed into `precision` (pair sums and their queries): plan with little scratch.  The
+ * plans otherwise take up to 4 GB of partial sums where that is faster; with the flag source
+ * splits take at most 256 MB (one split at least) and a both-sides sum at most 256 MB or 576 n
+ * bytes, and the schedules whose partial sums grow with n^2 (triangle, circle) are not taken.
+ * The query and the call must both carry it.  Results differ from those without the flag by
+ * the order of FP64 additions.  No counterpart in the reference. */
+#define VPM_COMPACT_WORKSPACE 0x200
 
 enum vpm_op {
   VPM_OP_SELFINDUCED_VELOCITY = 0,

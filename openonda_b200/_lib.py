@@ -138,6 +138,7 @@ def check(rc: int) -> None:
 
 
 UNIFORM_CORE = 0x100  # VPM_UNIFORM_CORE: every particle has the same core radius
+COMPACT_WORKSPACE = 0x200  # VPM_COMPACT_WORKSPACE: plan with little scratch
 
 
 def precision_code(precision: str, uniform_core: bool = False) -> int:

@@ -40,11 +40,11 @@ def rhs_vjp(x, a, sigma, nu, grad_u, grad_rate, precision="fp64"):
     ga = torch.empty((n, 3), dtype=_F64, device=dev)
     gs = torch.empty((n,), dtype=_F64, device=dev)
     gnu = None if v is None else torch.empty((n,), dtype=_F64, device=dev)
-    ws, _ = kernels._workspace(op, precision, n, n, dev)
+    ws, nb, code, _keep = kernels._scratch(op, _lib.precision_code(precision), n, n, dev)
     _lib.check(_lib.load().vpm_rhs_vjp(
         x.data_ptr(), a.data_ptr(), s.data_ptr(), kernels._ptr(v), n, gu.data_ptr(),
-        gr.data_ptr(), gx.data_ptr(), ga.data_ptr(), gs.data_ptr(), kernels._ptr(gnu),
-        _lib.precision_code(precision), ws.data_ptr(), ws.numel(), kernels._stream(dev)))
+        gr.data_ptr(), gx.data_ptr(), ga.data_ptr(), gs.data_ptr(), kernels._ptr(gnu), code, ws,
+        nb, kernels._stream(dev)))
     return gx, ga, gs, gnu
 
 
@@ -54,11 +54,11 @@ def kinetic_energy_grad(x, a, sigma, precision="fp64"):
     gx = torch.empty((n, 3), dtype=_F64, device=dev)
     ga = torch.empty((n, 3), dtype=_F64, device=dev)
     gs = torch.empty((n,), dtype=_F64, device=dev)
-    ws, _ = kernels._workspace("kinetic_energy_grad", precision, n, n, dev)
+    ws, nb, code, _keep = kernels._scratch("kinetic_energy_grad",
+                                           _lib.precision_code(precision), n, n, dev)
     _lib.check(_lib.load().vpm_kinetic_energy_grad(
         x.data_ptr(), a.data_ptr(), s.data_ptr(), n, gx.data_ptr(), ga.data_ptr(),
-        gs.data_ptr(), _lib.precision_code(precision), ws.data_ptr(), ws.numel(),
-        kernels._stream(dev)))
+        gs.data_ptr(), code, ws, nb, kernels._stream(dev)))
     return gx, ga, gs
 
 

@@ -111,6 +111,22 @@ struct Plan {
   int scalar = 0;  // FP64 scalar diagnostics with each unordered pair once (vpm_scalar.cuh)
 };
 
+// What a plan's partial sums may take.
+struct Budget {
+  size_t one_sided, both_sides;
+  bool compact;  // VPM_COMPACT_WORKSPACE: no triangle or circle, whose sets grow with n^2
+  // bytes: the caller's limit.  Compact plans stay within 256 MB, but may use four sets of the
+  // widest sums (18 values), the least the both-sides sweep works with.
+  Budget(bool compact, size_t bytes, int64_t n)
+      : one_sided(bytes), both_sides(bytes), compact(compact) {
+    if (!compact) return;
+    const size_t small = size_t(256) << 20, four = size_t(4 * 18 * 8) * size_t(n > 0 ? n : 0);
+    one_sided = bytes < small ? bytes : small;
+    const size_t both = small > four ? small : four;
+    both_sides = bytes < both ? bytes : both;
+  }
+};
+
 // FP32 self sums with at least this many particles evaluate each unordered pair once for both
 // particles (vpm_set_symmetric_min_n changes it).  Measured crossover of the fused sum:
 // one-sided 641 / 720 / 738 against both-sides 624 / 718 / 737 Gpairs/s at 16384 / 24576 /
@@ -1164,26 +1180,27 @@ struct CircleSweep {
 // (p->circle or p->pairs set).  MULTI: from the threshold on the sum takes the triangle, and the
 // many-launch sweep past the triangle's budget; otherwise the circle at all sizes its sets fit.
 template <class Op, bool MULTI>
-int plan_both64(int64_t m, int64_t n, Plan* p, size_t mpb) {
+int plan_both64(int64_t m, int64_t n, Plan* p, const Budget& b) {
   if (m != n) return VPM_OK;
+  const size_t mpb = b.both_sides;
   const bool large = RotSweep<Op>::usable(m, n, mpb);
-  if (n > 0 && n >= circle_min_n() && n < (int64_t(1) << 30) && RotSweep<Op>::tiles(n) >= 2 &&
-      !(MULTI && n >= g_sym_min_n.load())) {
+  if (!b.compact && n > 0 && n >= circle_min_n() && n < (int64_t(1) << 30) &&
+      RotSweep<Op>::tiles(n) >= 2 && !(MULTI && n >= g_sym_min_n.load())) {
     int rc = CircleSweep<Op>::plan(n, p, mpb);
     if (rc || p->circle) return rc;
   }
   if (!large) return VPM_OK;
   int rc = RotSweep<Op>::plan(n, p, mpb);
-  if (!rc && MULTI) rc = TriSweep<Op>::plan(n, p, mpb);
+  if (!rc && MULTI && !b.compact) rc = TriSweep<Op>::plan(n, p, mpb);
   return rc;
 }
 
 // The FP32 both-sides plan of a self sum: the many-launch sweep's, and the one-launch form where
 // its partial sums fit.
 template <class Op>
-int plan_both32(int64_t n, Plan* p, size_t mpb) {
-  int rc = RotSweep<Op>::plan(n, p, mpb);
-  if (!rc) rc = TriSweep<Op>::plan(n, p, mpb);
+int plan_both32(int64_t n, Plan* p, const Budget& b) {
+  int rc = RotSweep<Op>::plan(n, p, b.both_sides);
+  if (!rc && !b.compact) rc = TriSweep<Op>::plan(n, p, b.both_sides);
   return rc;
 }
 
@@ -1325,15 +1342,18 @@ struct Ops {
 bool is_probe(int op) { return op == VPM_OP_INDUCED_VELOCITY_AT || op == VPM_OP_VORTICITY_FIELD_AT; }
 
 template <class T, bool REFINE, bool UC = false>
-int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes) {
+int plan_op(int op, int64_t m, int64_t n, Plan* p, bool compact,
+            size_t max_partial_bytes = kMaxPartialBytes) {
   using O = Ops<T, REFINE, UC>;
+  const Budget b(compact, max_partial_bytes, n);
+  const size_t mpb = b.one_sided;
   switch (op) {
     case VPM_OP_SELFINDUCED_VELOCITY:
       if constexpr (LaneTraits<T>::kLanes == 2) {
-        if (RotSweep<typename O::VelBoth>::usable(m, n, mpb))
-          return plan_both32<typename O::VelBoth>(n, p, mpb);
+        if (RotSweep<typename O::VelBoth>::usable(m, n, b.both_sides))
+          return plan_both32<typename O::VelBoth>(n, p, b);
       } else {
-        const int rc = plan_both64<typename O::VelBoth64, true>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::VelBoth64, true>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::Vel, T, FIN_VEL>(m, n, p, mpb);
@@ -1348,16 +1368,16 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
       return plan_vector<typename O::VortAt, T, FIN_VORT>(m, n, p, mpb);
     case VPM_OP_STRENGTH_GRADIENTS:
       if constexpr (LaneTraits<T>::kLanes == 1) {
-        const int rc = plan_both64<typename O::StretchBoth64, false>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::StretchBoth64, false>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::Stretch, T, FIN_STRETCH>(m, n, p, mpb);
     case VPM_OP_STRENGTH_GRADIENTS_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
-        if (RotSweep<typename O::PseBoth>::usable(m, n, mpb))
-          return plan_both32<typename O::PseBoth>(n, p, mpb);
+        if (RotSweep<typename O::PseBoth>::usable(m, n, b.both_sides))
+          return plan_both32<typename O::PseBoth>(n, p, b);
       } else {
-        const int rc = plan_both64<typename O::PseBoth64, true>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::PseBoth64, true>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::Pse, T, FIN_PSE>(m, n, p, mpb);
@@ -1373,7 +1393,7 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
       return Sweep<typename O::Ens, T>::plan(m, n, p, mpb, true);
     case VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
-        if (RotSweep<typename O::VelStretchBoth>::usable(m, n, mpb)) {
+        if (RotSweep<typename O::VelStretchBoth>::usable(m, n, b.both_sides)) {
           // two builds of the fused sum on 768-particle tiles (3 and 2 resident CTAs per SM):
           // take the one whose launches fill the waves better, the 2-CTA build on a tie (it
           // measured equal or faster whenever its waves were as full).  A third on
@@ -1384,8 +1404,8 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
           constexpr double kSmallTileRate = 0.92;
           Plan pa, pb, pc;
           double ea = 0.0, eb = 0.0, ec = 0.0;
-          int rc = RotSweep<typename O::VelStretchBoth>::plan(n, &pa, mpb, &ea);
-          if (!rc) rc = RotSweep<typename O::VelStretchBothAlt>::plan(n, &pb, mpb, &eb);
+          int rc = RotSweep<typename O::VelStretchBoth>::plan(n, &pa, b.both_sides, &ea);
+          if (!rc) rc = RotSweep<typename O::VelStretchBothAlt>::plan(n, &pb, b.both_sides, &eb);
           if (rc) return rc;
           double e = ea;
           if (eb >= ea - 0.01) {
@@ -1395,8 +1415,8 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
           } else {
             *p = pa;
           }
-          if (RotSweep<typename O::VelStretchBothSmall>::usable(m, n, mpb)) {
-            rc = RotSweep<typename O::VelStretchBothSmall>::plan(n, &pc, mpb, &ec);
+          if (RotSweep<typename O::VelStretchBothSmall>::usable(m, n, b.both_sides)) {
+            rc = RotSweep<typename O::VelStretchBothSmall>::plan(n, &pc, b.both_sides, &ec);
             if (rc) return rc;
             if (kSmallTileRate * ec > e + 0.01) {
               pc.variant = 2;
@@ -1405,38 +1425,40 @@ int plan_op(int op, int64_t m, int64_t n, Plan* p, size_t mpb = kMaxPartialBytes
           }
           // the one-launch form of the same tiles (the same FP32 sums); of the two builds on
           // 768-particle tiles the one for 2 CTAs per SM
-          return p->variant == 2 ? TriSweep<typename O::VelStretchBothSmall>::plan(n, p, mpb)
-                                 : TriSweep<typename O::VelStretchBothAlt>::plan(n, p, mpb);
+          if (b.compact) return VPM_OK;
+          return p->variant == 2
+                     ? TriSweep<typename O::VelStretchBothSmall>::plan(n, p, b.both_sides)
+                     : TriSweep<typename O::VelStretchBothAlt>::plan(n, p, b.both_sides);
         }
       } else {
-        const int rc = plan_both64<typename O::VelStretchBoth64, true>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::VelStretchBoth64, true>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return plan_vector<typename O::VelStretch, T, FIN_VELSTRETCH>(m, n, p, mpb);
     case VPM_OP_LES_STEP_SUMS:
       if constexpr (LaneTraits<T>::kLanes == 2) {
-        if (RotSweep<typename O::LesStepBoth>::usable(m, n, mpb))
-          return plan_both32<typename O::LesStepBoth>(n, p, mpb);
+        if (RotSweep<typename O::LesStepBoth>::usable(m, n, b.both_sides))
+          return plan_both32<typename O::LesStepBoth>(n, p, b);
       } else {
-        const int rc = plan_both64<typename O::LesStepBoth64, true>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::LesStepBoth64, true>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return Sweep<typename O::LesStep, T>::plan(m, n, p, mpb);
     case VPM_OP_RHS_VJP:
       if constexpr (LaneTraits<T>::kLanes == 2) {
-        if (RotSweep<typename O::RhsVjpBoth>::usable(m, n, mpb))
-          return plan_both32<typename O::RhsVjpBoth>(n, p, mpb);
+        if (RotSweep<typename O::RhsVjpBoth>::usable(m, n, b.both_sides))
+          return plan_both32<typename O::RhsVjpBoth>(n, p, b);
       } else {
-        const int rc = plan_both64<typename O::RhsVjpBoth64, false>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::RhsVjpBoth64, false>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return Sweep<typename O::RhsVjp, T>::plan(m, n, p, mpb);
     case VPM_OP_RHS_VJP_PSE:
       if constexpr (LaneTraits<T>::kLanes == 2) {
-        if (RotSweep<typename O::RhsVjpPseBoth>::usable(m, n, mpb))
-          return plan_both32<typename O::RhsVjpPseBoth>(n, p, mpb);
+        if (RotSweep<typename O::RhsVjpPseBoth>::usable(m, n, b.both_sides))
+          return plan_both32<typename O::RhsVjpPseBoth>(n, p, b);
       } else {
-        const int rc = plan_both64<typename O::RhsVjpPseBoth64, false>(m, n, p, mpb);
+        const int rc = plan_both64<typename O::RhsVjpPseBoth64, false>(m, n, p, b);
         if (rc || p->circle || p->pairs) return rc;
       }
       return Sweep<typename O::RhsVjpPse, T>::plan(m, n, p, mpb);
@@ -1477,9 +1499,9 @@ Layout layout_for(int op, const Plan& p, int64_t m, int64_t n) {
 }
 
 template <class T, bool REFINE, bool UC = false>
-int workspace_for(int op, int64_t m, int64_t n, Layout* L, Plan* p,
+int workspace_for(int op, int64_t m, int64_t n, Layout* L, Plan* p, bool compact,
                   size_t max_partial_bytes = kMaxPartialBytes) {
-  int rc = plan_op<T, REFINE, UC>(op, m, n, p, max_partial_bytes);
+  int rc = plan_op<T, REFINE, UC>(op, m, n, p, compact, max_partial_bytes);
   if (rc) return rc;
   *L = layout_for<T>(op, *p, m, n);
   return VPM_OK;
@@ -1503,6 +1525,7 @@ struct Call {
   const void* records = nullptr;  // pre-packed sources (self sums); null = pack from AoS
   int64_t tgt_begin = 0;          // self sums: targets are records[tgt_begin, tgt_begin + m)
   size_t max_partial_bytes = kMaxPartialBytes;  // caps the source splits of the plan
+  bool compact = false;                         // VPM_COMPACT_WORKSPACE
   double* out3 = nullptr;  // VPM_OP_LES_STEP_SUMS: vorticity (m,3)
   double* out4 = nullptr;  // VPM_OP_LES_STEP_SUMS: enstrophy (device scalar)
   const double* aux = nullptr;  // VPM_OP_LES_TEST_FILTER: the filtered fields (n,3)
@@ -1552,7 +1575,7 @@ int run(const Call& c) {
 
   Plan p;
   Layout L;
-  rc = workspace_for<T, REFINE, UC>(c.op, c.m, c.n, &L, &p, c.max_partial_bytes);
+  rc = workspace_for<T, REFINE, UC>(c.op, c.m, c.n, &L, &p, c.compact, c.max_partial_bytes);
   if (rc) return rc;
   if (c.ws == nullptr) return fail(VPM_ERR_WORKSPACE, "workspace is null");
   if (reinterpret_cast<uintptr_t>(c.ws) % kAlign != 0)
@@ -1848,7 +1871,7 @@ int run_filter(const Call& c) {
   if (c.n == 0) return VPM_OK;
   Plan p;
   Layout L;
-  rc = workspace_for<T, REFINE>(c.op, c.n, c.n, &L, &p, c.max_partial_bytes);
+  rc = workspace_for<T, REFINE>(c.op, c.n, c.n, &L, &p, c.compact, c.max_partial_bytes);
   if (rc) return rc;
   if (c.ws == nullptr) return fail(VPM_ERR_WORKSPACE, "workspace is null");
   if (reinterpret_cast<uintptr_t>(c.ws) % kAlign != 0)
@@ -1868,6 +1891,9 @@ int run_filter(const Call& c) {
   return finalize<5>(part, p.splits, c.n, SetsFinalizeFilter{c.out, c.out2}, c.st);
 }
 
+// Flags of a precision code.
+constexpr int kPrecisionFlags = VPM_UNIFORM_CORE | VPM_COMPACT_WORKSPACE;
+
 // Decoded precision code: compute type, Newton-refined rsqrt, uniform cores.
 template <class T, bool REFINE, bool UC>
 struct Prec {
@@ -1878,7 +1904,7 @@ struct Prec {
 template <class F>
 int with_precision(int precision, F&& f) {
   const bool uc = (precision & VPM_UNIFORM_CORE) != 0;
-  switch (precision & ~VPM_UNIFORM_CORE) {
+  switch (precision & ~kPrecisionFlags) {
     case VPM_FP64:
       return uc ? f(Prec<double, false, true>{}) : f(Prec<double, false, false>{});
     case VPM_FP32C:
@@ -1890,7 +1916,8 @@ int with_precision(int precision, F&& f) {
   }
 }
 
-int dispatch(const Call& c, int precision) {
+int dispatch(Call c, int precision) {
+  c.compact = (precision & VPM_COMPACT_WORKSPACE) != 0;
   if (c.n < 0 || c.m < 0) return fail(VPM_ERR_ARG, "negative size");
   if (c.records) {
     if (is_probe(c.op)) return fail(VPM_ERR_ARG, "record entry points are for self sums");
@@ -1925,6 +1952,7 @@ struct GradCall {
   void* ws;
   size_t ws_bytes;
   cudaStream_t st;
+  bool compact = false;  // VPM_COMPACT_WORKSPACE
 };
 
 template <class T, bool REFINE>
@@ -1935,7 +1963,7 @@ int run_grad(const GradCall& c) {
   if (c.n == 0) return VPM_OK;
   Plan p;
   Layout L;
-  rc = workspace_for<T, REFINE>(c.op, c.n, c.n, &L, &p);
+  rc = workspace_for<T, REFINE>(c.op, c.n, c.n, &L, &p, c.compact);
   if (rc) return rc;
   if (c.ws == nullptr) return fail(VPM_ERR_WORKSPACE, "workspace is null");
   if (reinterpret_cast<uintptr_t>(c.ws) % kAlign != 0)
@@ -1997,8 +2025,9 @@ int run_grad(const GradCall& c) {
   return rc;
 }
 
-int dispatch_grad(const GradCall& c, int precision) {
-  precision &= ~VPM_UNIFORM_CORE;  // the adjoint keeps the general pair core
+int dispatch_grad(GradCall c, int precision) {
+  c.compact = (precision & VPM_COMPACT_WORKSPACE) != 0;
+  precision &= ~kPrecisionFlags;  // the adjoint keeps the general pair core
   if (c.n < 0) return fail(VPM_ERR_ARG, "negative size");
   if (c.n > 0 && (!c.pos || !c.str || !c.rad || !c.ox || !c.oa || !c.os))
     return fail(VPM_ERR_ARG, "null pointer");
@@ -2193,7 +2222,7 @@ template <class T, bool REFINE, bool UC, class F>
 int with_fused_both(int64_t n, F&& f) {
   using O = Ops<T, REFINE, UC>;
   Plan p;
-  int rc = plan_op<T, REFINE, UC>(VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS, n, n, &p);
+  int rc = plan_op<T, REFINE, UC>(VPM_OP_VELOCITY_AND_STRENGTH_GRADIENTS, n, n, &p, false);
   if (rc) return rc;
   if (!p.pairs)
     return fail(VPM_ERR_ARG, "n = " + std::to_string(n) +
@@ -2247,7 +2276,8 @@ size_t vpm_workspace_bytes(int op, int precision, int64_t m, int64_t n) {
     using Pp = decltype(P);
     Plan p;
     Layout L;
-    const int r = workspace_for<typename Pp::type, Pp::refine, Pp::uc>(op, m, n, &L, &p);
+    const int r = workspace_for<typename Pp::type, Pp::refine, Pp::uc>(
+        op, m, n, &L, &p, (precision & VPM_COMPACT_WORKSPACE) != 0);
     if (!r) total = L.total;
     return r;
   });
@@ -2332,7 +2362,7 @@ int vpm_finalize_pairs_partial(int op, const double* rows, const void* records,
   static_assert(OpVelStretchBoth<false, false>::NV == 9 && OpVelStretchBoth64<false>::NV == 9,
                 "the fused sum's 9 values per row");
   const unsigned blocks = unsigned((m + 255) / 256);
-  switch (precision & ~VPM_UNIFORM_CORE) {
+  switch (precision & ~kPrecisionFlags) {
     case VPM_FP64:
       finalize_rows_kernel<double, FIN_VELSTRETCH, 9><<<blocks, 256, 0, st>>>(
           rows, m, static_cast<const Rec<double>*>(records) + target_begin, out, out2);
@@ -2356,7 +2386,8 @@ int vpm_plan_info(int op, int precision, int64_t m, int64_t n, int64_t* target_b
   Plan p;
   const int rc = with_precision(precision, [&](auto P) {
     using Pp = decltype(P);
-    return plan_op<typename Pp::type, Pp::refine, Pp::uc>(op, m, n, &p);
+    return plan_op<typename Pp::type, Pp::refine, Pp::uc>(
+        op, m, n, &p, (precision & VPM_COMPACT_WORKSPACE) != 0);
   });
   if (rc) return rc;
   if (target_blocks) *target_blocks = p.tblocks;
@@ -2457,7 +2488,8 @@ int64_t vpm_sweep_launches(int op, int precision, int64_t m, int64_t n) {
   Plan p;
   const int rc = with_precision(precision, [&](auto P) {
     using Pp = decltype(P);
-    return plan_op<typename Pp::type, Pp::refine, Pp::uc>(op, m, n, &p);
+    return plan_op<typename Pp::type, Pp::refine, Pp::uc>(
+        op, m, n, &p, (precision & VPM_COMPACT_WORKSPACE) != 0);
   });
   if (rc) return -1;
   if (p.triangle) {  // zero the diagonal tiles' sets, those tiles, the triangle, finalize
@@ -2496,7 +2528,8 @@ int vpm_les_test_filter(const double* positions, const double* strengths,
          test_vorticity, test_filtered, 0, workspace, workspace_bytes,
          static_cast<cudaStream_t>(stream)};
   c.aux = fields;
-  switch (precision & ~VPM_UNIFORM_CORE) {
+  c.compact = (precision & VPM_COMPACT_WORKSPACE) != 0;
+  switch (precision & ~kPrecisionFlags) {
     case VPM_FP64:
       return run_filter<double, false>(c);
     case VPM_FP32C:
@@ -2509,7 +2542,7 @@ int vpm_les_test_filter(const double* positions, const double* strengths,
 }
 
 size_t vpm_record_bytes(int precision) {
-  switch (precision & ~VPM_UNIFORM_CORE) {
+  switch (precision & ~kPrecisionFlags) {
     case VPM_FP64:
       return sizeof(Rec<double>);
     case VPM_FP32C:
@@ -2533,7 +2566,7 @@ int vpm_pack_records(const double* positions, const double* strengths, const dou
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool uc = (precision & VPM_UNIFORM_CORE) != 0;
-  precision &= ~VPM_UNIFORM_CORE;
+  precision &= ~kPrecisionFlags;
   if (precision == VPM_FP64)
     return pack<double>(positions, strengths, radii, viscosities, n,
                         static_cast<Rec<double>*>(records), st, uc);

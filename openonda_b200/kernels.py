@@ -102,20 +102,25 @@ def plan_info(op: str, precision: str, m: int, n: int, uniform_core: bool = Fals
                 targets_per_thread=r.value)
 
 
-def _workspace(op, precision, m, n, dev, uniform_core=False):
-    nbytes = workspace_bytes(op, precision, m, n, uniform_core)
-    return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev), nbytes
-
-
 def _scratch(op, code, m, n, dev):
-    """Scratch of a sum with the precision code ``code``: (pointer, bytes, tensor)."""
-    nbytes = _lib.load().vpm_workspace_bytes(_lib.OPS[op], code, m, n)
+    """Scratch of a sum with the precision code ``code``: (pointer, bytes, code, tensor).  Where
+    the memory for it is not free, that of the sum's compact plan; the code says which."""
+    lib = _lib.load()
+    nbytes = lib.vpm_workspace_bytes(_lib.OPS[op], code, m, n)
     if nbytes == 0 and m > 0 and n > 0:
-        msg = _lib.load().vpm_last_error()
+        msg = lib.vpm_last_error()
         raise _lib.VPMError(_lib.VPM_ERR_CUDA, msg.decode() if msg else "workspace query failed")
     nbytes = max(nbytes, 256)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    return ws.data_ptr(), nbytes, ws
+    try:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    except torch.cuda.OutOfMemoryError:
+        small = code | _lib.COMPACT_WORKSPACE
+        less = lib.vpm_workspace_bytes(_lib.OPS[op], small, m, n)
+        if not 0 < less < nbytes:
+            raise
+        code, nbytes = small, less
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    return ws.data_ptr(), nbytes, code, ws
 
 
 def _self_inputs(positions, strengths, radii):
@@ -136,7 +141,7 @@ def selfinduced_velocity(positions, strengths, radii, precision="fp64", uniform_
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     out = _out(x)
     code = _lib.precision_code(precision, uniform_core)
-    ws, nb, _keep = _scratch("selfinduced_velocity", code, n, n, dev)
+    ws, nb, code, _keep = _scratch("selfinduced_velocity", code, n, n, dev)
     _lib.check(_lib.load().vpm_selfinduced_velocity(
         x.data_ptr(), a.data_ptr(), s.data_ptr(), n, out.data_ptr(), code, ws, nb,
         _stream(dev)))
@@ -147,7 +152,7 @@ def strength_gradients(positions, strengths, radii, precision="fp64", uniform_co
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     out = _out(x)
     code = _lib.precision_code(precision, uniform_core)
-    ws, nb, _keep = _scratch("strength_gradients", code, n, n, dev)
+    ws, nb, code, _keep = _scratch("strength_gradients", code, n, n, dev)
     _lib.check(_lib.load().vpm_strength_gradients(
         x.data_ptr(), a.data_ptr(), s.data_ptr(), n, out.data_ptr(), code, ws, nb,
         _stream(dev)))
@@ -159,7 +164,7 @@ def velocity_and_strength_gradients(positions, strengths, radii,
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     u, g = _out(x), _out(x)
     code = _lib.precision_code(precision, uniform_core)
-    ws, nb, _keep = _scratch("velocity_and_strength_gradients", code, n, n, dev)
+    ws, nb, code, _keep = _scratch("velocity_and_strength_gradients", code, n, n, dev)
     _lib.check(_lib.load().vpm_velocity_and_strength_gradients(
         x.data_ptr(), a.data_ptr(), s.data_ptr(), n, u.data_ptr(), g.data_ptr(), code, ws, nb,
         _stream(dev)))
@@ -176,12 +181,11 @@ def les_step_sums(positions, strengths, radii, ref_extra_4pi=True,
     g = torch.empty((n, 3), dtype=_F64, device=dev)
     w = torch.empty((n, 3), dtype=_F64, device=dev)
     e = torch.empty((), dtype=_F64, device=dev)
-    ws, nb = _workspace("les_step_sums", precision, n, n, dev, uniform_core)
+    code = _lib.precision_code(precision, uniform_core)
+    ws, nb, code, _keep = _scratch("les_step_sums", code, n, n, dev)
     _lib.check(_lib.load().vpm_les_step_sums(
         _ptr(x), _ptr(a), _ptr(s), n, _ptr(u), _ptr(g), _ptr(w), _ptr(e),
-        int(bool(ref_extra_4pi)),
-        _lib.precision_code(precision, uniform_core), _ptr(ws), ws.numel(),
-        _stream(dev)))
+        int(bool(ref_extra_4pi)), code, ws, nb, _stream(dev)))
     return u, g, w, e
 
 
@@ -194,10 +198,9 @@ def les_test_filter(positions, strengths, test_radii, fields, precision="fp64"):
     _same_device(x, f)
     w = torch.empty((n, 3), dtype=_F64, device=dev)
     fh = torch.empty((n, 3), dtype=_F64, device=dev)
-    ws, nb = _workspace("les_test_filter", precision, n, n, dev)
+    ws, nb, code, _keep = _scratch("les_test_filter", _lib.precision_code(precision), n, n, dev)
     _lib.check(_lib.load().vpm_les_test_filter(
-        _ptr(x), _ptr(a), _ptr(s), _ptr(f), n, _ptr(w), _ptr(fh),
-        _lib.precision_code(precision), _ptr(ws), ws.numel(), _stream(dev)))
+        _ptr(x), _ptr(a), _ptr(s), _ptr(f), n, _ptr(w), _ptr(fh), code, ws, nb, _stream(dev)))
     return w, fh
 
 
@@ -208,7 +211,7 @@ def strength_gradients_pse(positions, strengths, radii, viscosities,
     _same_device(x, v)
     out = _out(x)
     code = _lib.precision_code(precision, uniform_core)
-    ws, nb, _keep = _scratch("strength_gradients_pse", code, n, n, dev)
+    ws, nb, code, _keep = _scratch("strength_gradients_pse", code, n, n, dev)
     _lib.check(_lib.load().vpm_strength_gradients_pse(
         x.data_ptr(), a.data_ptr(), s.data_ptr(), v.data_ptr(), n, out.data_ptr(), code, ws, nb,
         _stream(dev)))
@@ -222,7 +225,7 @@ def _probe(fn_name, op, targets, positions, strengths, radii, precision):
     m = t.shape[0]
     out = _out(t)
     code = _lib.precision_code(precision)
-    ws, nb, _keep = _scratch(op, code, m, n, dev)
+    ws, nb, code, _keep = _scratch(op, code, m, n, dev)
     fn = getattr(_lib.load(), fn_name)
     _lib.check(fn(t.data_ptr(), m, x.data_ptr(), a.data_ptr(), s.data_ptr(), n, out.data_ptr(),
                   code, ws, nb, _stream(dev)))
@@ -242,20 +245,20 @@ def vorticity_field_at(targets, positions, strengths, radii, precision="fp64"):
 def total_kinetic_energy(positions, strengths, radii, precision="fp64"):
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     out = torch.empty((), dtype=_F64, device=dev)
-    ws, nb = _workspace("total_kinetic_energy", precision, n, n, dev)
+    code = _lib.precision_code(precision)
+    ws, nb, code, _keep = _scratch("total_kinetic_energy", code, n, n, dev)
     _lib.check(_lib.load().vpm_total_kinetic_energy(
-        _ptr(x), _ptr(a), _ptr(s), n, _ptr(out), _lib.precision_code(precision), _ptr(ws),
-        ws.numel(), _stream(dev)))
+        _ptr(x), _ptr(a), _ptr(s), n, _ptr(out), code, ws, nb, _stream(dev)))
     return out
 
 
 def total_helicity(positions, strengths, radii, ref_extra_4pi=True, precision="fp64"):
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     out = torch.empty((), dtype=_F64, device=dev)
-    ws, nb = _workspace("total_helicity", precision, n, n, dev)
+    ws, nb, code, _keep = _scratch("total_helicity", _lib.precision_code(precision), n, n, dev)
     _lib.check(_lib.load().vpm_total_helicity(
-        _ptr(x), _ptr(a), _ptr(s), n, int(bool(ref_extra_4pi)), _ptr(out),
-        _lib.precision_code(precision), _ptr(ws), ws.numel(), _stream(dev)))
+        _ptr(x), _ptr(a), _ptr(s), n, int(bool(ref_extra_4pi)), _ptr(out), code, ws, nb,
+        _stream(dev)))
     return out
 
 
@@ -263,10 +266,11 @@ def total_enstrophy(positions, strengths, radii, ref_extra_4pi=True,
                     precision="fp64", uniform_core=False):
     x, a, s, n, dev = _self_inputs(positions, strengths, radii)
     out = torch.empty((), dtype=_F64, device=dev)
-    ws, nb = _workspace("total_enstrophy", precision, n, n, dev, uniform_core)
+    code = _lib.precision_code(precision, uniform_core)
+    ws, nb, code, _keep = _scratch("total_enstrophy", code, n, n, dev)
     _lib.check(_lib.load().vpm_total_enstrophy(
-        _ptr(x), _ptr(a), _ptr(s), n, int(bool(ref_extra_4pi)), _ptr(out),
-        _lib.precision_code(precision, uniform_core), _ptr(ws), ws.numel(), _stream(dev)))
+        _ptr(x), _ptr(a), _ptr(s), n, int(bool(ref_extra_4pi)), _ptr(out), code, ws, nb,
+        _stream(dev)))
     return out
 
 
