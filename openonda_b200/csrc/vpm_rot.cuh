@@ -183,6 +183,14 @@ struct RotStd {
   using Lane = RotSrc;
   static constexpr int kP = 2;
   static constexpr bool kSrcCore = !UC;  // the pair core needs the source's sigma
+  // Whether rot_sweep_kernel has a batch written out in its own body instead of calling
+  // rot_batch and rot_combine: the same operations in the same order, which the compiler
+  // schedules differently.  Written out where that is the faster form; written out / called at
+  // 160000 particles (ms, general cores then uniform): velocity 13.74 / 13.89 and 12.66 / 12.44,
+  // refined 15.30 / 15.28 and 13.97 / 14.28; PSE 10.99 / 11.16 and 10.17 / 10.15, refined 12.53 /
+  // 12.45 and 11.60 / 11.53; fused 26.26 / 26.26 and 25.10 / 25.07; LES 40.43 / 40.26 and 34.77 /
+  // 34.79; adjoint 60.27 / 60.34, with PSE 89.83 / 89.82.
+  static constexpr bool kOpenBatch = false;
 
   // Source j of the packed records (j < n), or a padding source far away with no strength.
   __device__ __forceinline__ static Lane load_lane(const Record* rec, int64_t j, int64_t n) {
@@ -345,6 +353,7 @@ struct OpVelBoth : RotStd<OpVel<float2, REFINE, UC>, UC> {
   using V = float2;
   static constexpr int NV = 3;
   static constexpr int kP = VPM_ROT3_P;
+  static constexpr bool kOpenBatch = REFINE == UC;
   static constexpr int kMinBlocks = VPM_ROT3_MINB;
   static constexpr int kUnroll = VPM_ROT_UNROLL;
   static constexpr int kSrcWindow = VPM_ROT3_SRC_WINDOW;
@@ -445,6 +454,7 @@ struct OpPseBoth : RotStd<OpPse<float2, REFINE, UC>, UC> {
   using V = float2;
   static constexpr int NV = 3;
   static constexpr int kP = VPM_ROT3_P;
+  static constexpr bool kOpenBatch = !REFINE && !UC;
   static constexpr int kMinBlocks = VPM_ROT3_MINB;
   static constexpr int kUnroll = VPM_ROT_UNROLL;
   static constexpr int kSrcWindow = VPM_ROT3_SRC_WINDOW;
@@ -656,6 +666,7 @@ struct OpRhsVjpBoth {
   };
   static constexpr int kLaneValues = PSE ? 17 : 16;  // values that move around the warp
   static constexpr int NV = OneSided::NV;
+  static constexpr bool kOpenBatch = !REFINE && !PSE;  // (see RotStd)
   static constexpr int kP = PSE ? VPM_ROTGP_P : VPM_ROTG_P;
   static constexpr int kMinBlocks = PSE ? VPM_ROTGP_MINB : VPM_ROTG_MINB;
   static constexpr int kUnroll = PSE ? VPM_ROTGP_UNROLL : VPM_ROTG_UNROLL;
@@ -1050,8 +1061,72 @@ rot_sweep_kernel(const RotArgs a) {
   const int nb = (cnt + 31) / 32;
   Lane nxt = Op::load_lane(rec, j0 + lane, j0 + cnt);
   for (int b = 0; b < nb; ++b) {
-    const Lane cur = nxt;  // the source this lane holds at step 0
+    Lane cur = nxt;  // the source this lane holds at step 0
     if (b + 1 < nb) nxt = Op::load_lane(rec, j0 + (b + 1) * 32 + lane, j0 + cnt);
+    if constexpr (!DIAG && Op::kOpenBatch) {
+      // rot_batch and rot_combine, written out (see RotStd::kOpenBatch)
+      constexpr int WT = kRotWarps * 32;
+      constexpr int SW = Op::kSrcWindow;
+      constexpr int TW = Op::kTgtWindow, TWS = Op::kTgtWindowShort, TWL = Op::kTgtWindowLong;
+      float2 jv[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) jv[v] = make_float2(0.f, 0.f);
+      float2* jb = jbuf + (b % Op::kJBufs) * (NJ * WT);
+      const int src_lane = (lane + 1) & 31;
+      for (int w = 0; w < 32 / SW; ++w) {
+#pragma unroll Op::kUnroll
+        for (int st = 0; st < SW; ++st) {
+          const typename Op::SrcT src = Op::broadcast(cur);
+#pragma unroll
+          for (int p = 0; p < P; ++p) Op::pair2(tg[p], acc[p], jv, src);
+          Op::shuffle(cur, src_lane);
+          if (st != SW - 1) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              if (Op::carried(v)) {
+                jv[v].x = __shfl_sync(0xffffffffu, jv[v].x, src_lane);
+                jv[v].y = __shfl_sync(0xffffffffu, jv[v].y, src_lane);
+              }
+            }
+          }
+        }
+        const int slot = warp * 32 + ((lane + (w + 1) * SW - 1) & 31);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          if (Op::carried(v)) {
+            float2* e = jb + v * WT + slot;
+            *e = (w == 0) ? jv[v] : (*e + jv[v]);
+            jv[v] = make_float2(0.f, 0.f);
+          }
+        }
+        const int done = (w + 1) * SW;  // steps of this batch done
+        const bool at_full = done % TW == 0;
+        const bool at_short = TWS > 0 && done % (TWS > 0 ? TWS : 1) == 0;
+        const bool at_long = TWL > 0 && (b * 32 + done) % (TWL > 0 ? TWL : 1) == 0;
+        if (at_full || at_short || at_long)
+          rot_fold<Op, false>(car, acc, lt, [&](int v) {
+            return (TWL > 0 && Op::long_fold(v))    ? at_long
+                   : (TWS > 0 && Op::short_fold(v)) ? at_short
+                                                    : at_full;
+          });
+      }
+      __syncthreads();  // the batch's source-side sums are complete
+      const int nsrc = (cnt - b * 32 < 32) ? cnt - b * 32 : 32;
+      for (int q = tid; q < 32 * NJ; q += kRotThreads) {
+        const int v = q >> 5, jj = q & 31;  // consecutive threads: consecutive sources
+        if (jj >= nsrc || !Op::carried(v)) continue;
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < kRotWarps; ++k) {
+          const float2 e = jb[v * WT + k * 32 + jj];
+          sum += double(e.x);
+          sum += double(e.y);
+        }
+        atomicAdd(&a.acc[(int64_t(set_j) * NV + v) * a.n + (j0 + b * 32 + jj)], -sum);
+      }
+      if constexpr (Op::kJBufs == 1) __syncthreads();
+      continue;
+    }
     float2* jb = jbuf + (b % Op::kJBufs) * (NJ * kRotWarps * 32);
     rot_batch<Op, DIAG>(cur, tg, acc, lt, car, jb, i0, j0 + b * 32, b, warp, lane);
     if constexpr (!DIAG) {
