@@ -1213,12 +1213,23 @@ int plan_both32(int64_t n, Plan* p, const Budget& b) {
 constexpr int64_t kSmallSources = 4096;
 template <class T>
 constexpr int64_t small_pairs = LaneTraits<T>::kLanes == 1 ? 6000000 : 16000000;
+// Most blocks of targets (32 per lane).  Past it the limit on pairs leaves fewer than 62 sources:
+// one or two windows for the four warps of a block, the others idle.  Probe sums, us, three
+// launches / one (velocity, vorticity): FP64 131072 x 40 21.9 / 25.9 and 20.3 / 26.2, 300000 x 10
+// 21.3 / 31.8 and 20.3 / 32.0, 10^6 x 1 38.9 / 75.0; FP32c 300000 x 40 25.8 / 28.5 and 24.0 / 26.3,
+// 10^6 x 16 48.2 / 65.2.  Below it, FP64 62000 x 96 25.4 / 19.9, 50000 x 10 9.4 / 8.0, 10000 x 300
+// 34.2 / 17.0, 3000 x 2000 35.1 / 21.8; FP32c 250000 x 64 31.1 / 27.5, 100000 x 40 15.0 / 12.7,
+// 8000 x 2000 28.9 / 24.0.  (FP64 at 100000 targets and 1 to 40 sources: 9.4 to 19.8 / 9.8 to 20.5
+// on the device, and 29 / 14 to 23 for a call that is not captured.)
+template <class T>
+constexpr int64_t kSmallBlocks = LaneTraits<T>::kLanes == 1 ? 3200 : 4096;
 
 int64_t small_windows(int64_t n) { return (n + kSmallWindow - 1) / kSmallWindow; }
 
 template <class T>
 bool small_usable(int64_t m, int64_t n) {
-  return m > 0 && n > 0 && n < kSmallSources && m <= small_pairs<T> / n;
+  return m > 0 && n > 0 && n < kSmallSources && m <= small_pairs<T> / n &&
+         m <= kSmallBlocks<T> * 32 * LaneTraits<T>::kLanes;
 }
 
 template <class T, int KIND, int NV>
