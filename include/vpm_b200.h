@@ -176,7 +176,8 @@ int vpm_velocity_and_strength_gradients(const double* positions, const double* s
  * launch.  The diagonal tiles of the triangle, and of short launches, run on a second stream of
  * the library's, forked from and joined to the caller's stream by events inside the call, so
  * stream order and CUDA-graph capture see one call as before; that stream is created by the first
- * such call in a context (make it before any stream capture).  The FP64 self sums (those above,
+ * such call in a context (make it before any stream capture).  While it is part of one stream's
+ * capture, calls on other streams run those tiles on their own stream.  The FP64 self sums (those above,
  * the stretching and the adjoint among them) do so from a sixth of this value on, in one launch
  * over a circle of tiles; the stretching and the adjoint stay there while their partial sums fit
  * 4 GB.  The scalar diagnostics in FP64 take each unordered pair once at every size.  Sets the

@@ -567,6 +567,20 @@ int side_stream(SideStream** out) {
   return VPM_OK;
 }
 
+// Whether work of `st` can fork to the side stream.  It cannot while the side stream is part of
+// another stream's capture, which a call made before that capture ends would join and break; such
+// a call keeps its diagonal tiles on its own stream.  The calling thread holds g_side_mu.
+bool side_free(const SideStream& ss, cudaStream_t st) {
+  cudaStreamCaptureStatus side = cudaStreamCaptureStatusNone, own = side;
+  unsigned long long side_id = 0, own_id = 0;
+  cudaError_t e = cudaStreamGetCaptureInfo(ss.stream, &side, &side_id);
+  if (e == cudaSuccess && side == cudaStreamCaptureStatusNone) return true;
+  if (e == cudaSuccess) e = cudaStreamGetCaptureInfo(st, &own, &own_id);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess && side == cudaStreamCaptureStatusActive && own == side &&
+         own_id == side_id;
+}
+
 template <class Op>
 struct RotSweep {
   static constexpr int NV = Op::NV;
@@ -732,6 +746,7 @@ struct RotSweep {
     const int npairs = nt / 2;
     SideStream* ss = nullptr;
     std::unique_lock<std::mutex> lk(g_side_mu, std::defer_lock);
+    bool beside = false;
     if (p.diag_beside) {
       // the pair launches on the caller's stream, the diagonal tiles on the side stream into
       // sets [sets of the pairs, + kRotDiagSplit); the caller's stream waits for both (fork
@@ -739,7 +754,8 @@ struct RotSweep {
       lk.lock();
       rc = side_stream(&ss);
       if (rc) return rc;
-      e = cudaEventRecord(ss->fork, st);
+      beside = side_free(*ss, st);
+      if (beside) e = cudaEventRecord(ss->fork, st);
       if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord(fork)");
     } else {
       launch_kernel<true>(unsigned(nt * kRotDiagSplit), RotArgs{rec, n, nt, 0, acc}, st);
@@ -753,13 +769,14 @@ struct RotSweep {
       if (e != cudaSuccess) return cuda_fail(e, "both-sides sweep launch");
     }
     if (p.diag_beside) {
-      e = cudaStreamWaitEvent(ss->stream, ss->fork, 0);
+      if (beside) e = cudaStreamWaitEvent(ss->stream, ss->fork, 0);
       if (e != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent(fork)");
       RotArgs d{rec, n, nt, 0, acc};
       d.set0 = 2 * p.pairs;
-      launch_kernel<true>(unsigned(nt * kRotDiagSplit), d, ss->stream);
+      launch_kernel<true>(unsigned(nt * kRotDiagSplit), d, beside ? ss->stream : st);
       e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(e, "both-sides sweep launch");
+      if (!beside) return VPM_OK;
       e = cudaEventRecord(ss->join, ss->stream);
       if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord(join)");
       e = cudaStreamWaitEvent(st, ss->join, 0);
@@ -1067,11 +1084,14 @@ struct TriSweep {
       SideStream* ss = nullptr;
       rc = side_stream(&ss);
       if (rc) return rc;
-      cudaError_t e = cudaEventRecord(ss->fork, st);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(ss->stream, ss->fork, 0);
+      const bool beside = side_free(*ss, st);
+      cudaError_t e = cudaSuccess;
+      if (beside) e = cudaEventRecord(ss->fork, st);
+      if (beside && e == cudaSuccess) e = cudaStreamWaitEvent(ss->stream, ss->fork, 0);
       if (e != cudaSuccess) return cuda_fail(e, "side stream fork");
       RotSweep<Op>::template launch_kernel<true>(unsigned(l.nt * kRotDiagSplit),
-                                                 RotArgs{rec, n, l.nt, 0, acc}, ss->stream);
+                                                 RotArgs{rec, n, l.nt, 0, acc},
+                                                 beside ? ss->stream : st);
       e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(e, "both-sides sweep launch");
       const unsigned grid = unsigned(p.shares.blocks());
@@ -1084,8 +1104,8 @@ struct TriSweep {
       }
       e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(e, "triangle sweep launch");
-      e = cudaEventRecord(ss->join, ss->stream);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ss->join, 0);
+      if (beside) e = cudaEventRecord(ss->join, ss->stream);
+      if (beside && e == cudaSuccess) e = cudaStreamWaitEvent(st, ss->join, 0);
       if (e != cudaSuccess) return cuda_fail(e, "side stream join");
     }
     if (rc) return rc;
