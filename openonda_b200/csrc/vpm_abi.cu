@@ -1211,7 +1211,9 @@ int plan_both64(int64_t m, int64_t n, Plan* p, const Budget& b) {
   }
   if (!large) return VPM_OK;
   int rc = RotSweep<Op>::plan(n, p, mpb);
-  if (!rc && MULTI && !b.compact) rc = TriSweep<Op>::plan(n, p, mpb);
+  if constexpr (MULTI) {
+    if (!rc && !b.compact) rc = TriSweep<Op>::plan(n, p, mpb);
+  }
   return rc;
 }
 
