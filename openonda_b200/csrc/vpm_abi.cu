@@ -422,7 +422,7 @@ template <int NV, class Finalize>
 int finalize(const double* part, int splits, int64_t m, const Finalize& fin, cudaStream_t st) {
   if (m <= 0) return VPM_OK;
   if (splits >= kSetLanesMinSplits && m <= kSetLanesMaxTargets) {
-    finalize_sets_kernel<NV, NV, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
+    finalize_sets_kernel<NV, NoSourceSums, SplitSets><<<unsigned((m + 31) / 32), 32 * kSetLanes, 0, st>>>(
         part, SplitSets{splits}, m, fin);
   } else {
     const int threads = 256;
@@ -1110,7 +1110,7 @@ struct TriSweep {
     }
     if (rc) return rc;
     const TriSets sets{l, p.shares, kTile, kRotDiagSplit, n, source};
-    finalize_sets_kernel<NV, Op::kSymFrom, TriSets, Finalize>
+    finalize_sets_kernel<NV, SourceSums<Op>, TriSets, Finalize>
         <<<unsigned((n + 31) / 32), 32 * kSetLanes, 0, st>>>(acc, sets, n, fin);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");
@@ -1128,7 +1128,6 @@ int64_t circle_min_n() { return g_sym_min_n.load() / 6; }
 template <class Op>
 struct CircleSweep {
   static constexpr int NV = Op::NV;
-  static constexpr int NJ = Op::kSymFrom;
   static constexpr int kTile = rot_tile<Op>();
   static constexpr size_t kSmem = lists64_smem_bytes<Op>();
 
@@ -1188,7 +1187,7 @@ struct CircleSweep {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "circle sweep launch");
     const CircleSets sets{l, p.shares, kTile, tsets, n};
-    finalize_sets_kernel<NV, NJ, CircleSets, Finalize>
+    finalize_sets_kernel<NV, SourceSums<Op>, CircleSets, Finalize>
         <<<unsigned((n + 31) / 32), 32 * kSetLanes, 0, st>>>(acc, sets, n, fin);
     e = cudaGetLastError();
     return e == cudaSuccess ? VPM_OK : cuda_fail(e, "finalize launch");

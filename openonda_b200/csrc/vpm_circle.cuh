@@ -15,8 +15,9 @@
 //     begin the next;
 //   * nothing is accumulated in memory: for target tile I, source j's sums go to the set of the
 //     distance of their tiles, and a block's target sums to the set of its place among the
-//     blocks that share the list.  Every element that is read has been written exactly once, so
-//     no set is zeroed, and the finalize adds the sets in a fixed order.
+//     blocks that share the list.  Every element that is read has been written exactly once (the
+//     finalize passes by the values without source sums), so no set is zeroed, and the finalize
+//     adds the sets in a fixed order.
 //
 // A target past n (in the last tile) is a particle far away without strength, as a source past n
 // is: the pair's terms underflow to zero on both sides.

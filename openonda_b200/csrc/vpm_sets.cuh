@@ -2,7 +2,7 @@
 //
 // acc[set][value][n]: a block takes 32 particles, its kSetLanes warps sum the sets in turn (warp
 // q the sets q, q + kSetLanes, ..), the warps' sums are added in order and Finalize gets every
-// particle's NV sums.  One thread per particle (finalize_vec_kernel) walks the sets one after
+// particle's NV sums.  One thread per particle (finalize_kernel) walks the sets one after
 // another: with tens of sets and a few thousand particles it waits for memory most of the time
 // (FP64 adjoint of 1000 particles 80 -> 27 us with this pass and splits down to 64 sources).
 #pragma once
@@ -27,9 +27,20 @@ struct SplitSets {
   }
 };
 
+// The values with source sums: the others' places in a source set are never written.
+template <class Op>
+struct SourceSums {
+  __device__ __forceinline__ static constexpr bool has(int v) {
+    return v < Op::kSymFrom && Op::carried(v);
+  }
+};
+struct NoSourceSums {
+  __device__ __forceinline__ static constexpr bool has(int) { return false; }
+};
+
 // Sets: for particle i, t sets of target sums (all NV values, acc[set][value][n]) and s sets of
-// source sums (the first NJ values) where source_set says, its values `stride` apart.
-template <int NV, int NJ, class Sets, class Finalize>
+// source sums (the values that Sources has) where source_set says, its values `stride` apart.
+template <int NV, class Sources, class Sets, class Finalize>
 __global__ void __launch_bounds__(32 * kSetLanes)
 finalize_sets_kernel(const double* __restrict__ acc, const Sets sets, int64_t n,
                      const Finalize fin) {
@@ -53,7 +64,8 @@ finalize_sets_kernel(const double* __restrict__ acc, const Sets sets, int64_t n,
       int64_t stride = n;
       const double* p = sets.template source_set<NV>(acc, q, i, stride);
 #pragma unroll
-      for (int k = 0; k < NJ; ++k) v[k] += p[int64_t(k) * stride];
+      for (int k = 0; k < NV; ++k)
+        if (Sources::has(k)) v[k] += p[int64_t(k) * stride];
     }
   }
 #pragma unroll
