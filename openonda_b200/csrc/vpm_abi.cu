@@ -883,8 +883,10 @@ struct ScalarSweep {
     return VPM_OK;
   }
 
-  // partial: [p.splits][p.tblocks][2], within the plan's p.splits * n doubles (n > 1; one tile's
-  // two doubles fit the region's alignment)
+  // doubles of partial sums: [p.splits][p.tblocks][2] (the same for every operator)
+  static size_t partials(const Plan& p) { return size_t(p.splits) * size_t(p.tblocks) * 2; }
+
+  // partial: partials(p) doubles
   static int launch(const Plan& p, const Rec<double>* rec, int64_t n, double* partial,
                     double scale, double* out, cudaStream_t st) {
     const ScalarArgs a{rec, n, int(p.tblocks), int(p.chunk), partial};
@@ -1523,7 +1525,9 @@ Layout layout_for(int op, const Plan& p, int64_t m, int64_t n) {
   L.tgt_off = off;
   if (is_probe(op)) off = align_up(off + size_t(m > 0 ? m : 0) * sizeof(Rec<T>));
   L.part_off = off;
-  off = align_up(off + size_t(p.splits) * p.nv * size_t(m > 0 ? m : 0) * sizeof(double));
+  const size_t partials = p.scalar ? ScalarSweep<ScalarKe>::partials(p)
+                                   : size_t(p.splits) * p.nv * size_t(m > 0 ? m : 0);
+  off = align_up(off + partials * sizeof(double));
   L.scalar_off = off;
   if (op == VPM_OP_LES_STEP_SUMS) off = align_up(off + size_t(m > 0 ? m : 0) * sizeof(double));
   L.total = off;

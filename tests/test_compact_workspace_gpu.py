@@ -68,3 +68,13 @@ def test_little_free_memory(n):
     for k, (g, w) in enumerate(zip(got, want)):
         assert normwise(g.cpu().numpy(), w.cpu().numpy()) <= 1e-12, k
     assert kernels.device_errors() == 0
+
+
+@pytest.mark.parametrize("op", ["total_kinetic_energy", "total_helicity", "total_enstrophy"])
+def test_bytes_of_the_fp64_scalars(op):
+    """The FP64 diagnostics leave two doubles per block: their scratch is the packed records and
+    at most 256 splits of the tiles of 128 particles."""
+    for n in (1, 2, 1000, 32768, 1 << 20, 1 << 22):
+        records = 64 * n
+        assert records < _bytes(op, 0, n) <= records + 16 * 256 * -(-n // 128) + 512, n
+        assert _bytes(op, 0, n) <= records + (n << 3) + (1 << 20), n
