@@ -25,7 +25,8 @@
  *     the calling thread.  Inputs are never modified; nothing throws across the ABI.
  *   - The pair sums read all of their input arrays before they write an output, so an output
  *     may overlap the inputs (not the packed records of vpm_sweep_records).
- *   - Radii must be positive.  Results are deterministic for a given device and sizes.
+ *   - Radii must be positive.  A pair whose r^2 + core^2 is below 2^-1022 (FP64; 2^-126 in FP32)
+ *     counts as one at zero.  Results are deterministic for a given device and sizes.
  */
 #ifndef VPM_B200_H
 #define VPM_B200_H

@@ -88,13 +88,15 @@ __device__ __forceinline__ float2 rsqrt_lane(float2 x) {
 // FP64: the hardware seed (PTX rsqrt.approx.ftz.f64, a 21-bit significand) and one third-order
 // step of the binomial series for x^(-1/2) about the seed: with e = 1 - x y^2,
 //   x^(-1/2) = y (1 - e)^(-1/2) = y (1 + e/2 + 3 e^2/8 + O(e^3)).
-// y^2 is exact in FP64, so e carries one rounding.  Five FP64 operations and no branch, so the
-// chains of a thread's targets interleave: 946 -> 1966 G roots/s at 8 warps per SM against CUDA's
-// rsqrt(), 1712 -> 2116 at 64, and the same bits on 2^20 arguments from 2^-900 to 2^900.  In the
-// sweeps (Gpairs/s at 131072 particles): fused both-sides 447 -> 457, velocity 723 -> 743, PSE 898
-// -> 946, LES 231 -> 264, kinetic energy 476 -> 493.  Outside the normal positive numbers (zero,
-// subnormals, infinity, NaN, negative) the seed itself is the result: an integer compare and
-// select, off the FP64 pipe.
+// y^2 is exact in FP64, so e carries one rounding; the truncation is below 2^-60 and the result
+// within one unit in the last place (tests/test_fp64_root_gpu.py holds a sum that takes its fifth
+// power to that at 2^20 arguments).  Five FP64 operations and no branch, so the chains of a
+// thread's targets interleave: 946 -> 1966 G roots/s at 8 warps per SM against CUDA's rsqrt(), 1712
+// -> 2116 at 64.  In the sweeps (Gpairs/s at 131072 particles): fused both-sides 447 -> 457,
+// velocity 723 -> 743, PSE 898 -> 946, LES 231 -> 264, kinetic energy 476 -> 493.  Outside the
+// normal positive numbers the seed itself is the result (an integer compare and select, off the
+// FP64 pipe): infinity for zero, 0 for infinity, NaN for NaN and negative numbers.  Positive
+// subnormals count as zero, where rsqrt() gives their root (r^2 + core^2 below 2^-1022).
 __device__ __forceinline__ double rsqrt_fp64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
