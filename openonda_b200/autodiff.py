@@ -118,7 +118,7 @@ def kinetic_energy(x, a, sigma, precision="fp64"):
 
 def _axpy(x, k, c):
     """x + c k in one operation where c is a plain number (a tensor c keeps its gradient)."""
-    return torch.add(x, k, alpha=c) if isinstance(c, (int, float)) else x + c * k
+    return torch.add(x, k, alpha=float(c)) if isinstance(c, (int, float)) else x + c * k
 
 
 def _rk4_combine(x, k1, k2, k3, k4, dt):
