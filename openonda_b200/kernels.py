@@ -133,8 +133,9 @@ def _self_inputs(positions, strengths, radii):
 
 
 def _out(x):
-    """A new (n, 3) result like the contiguous positions x."""
-    return torch.empty_like(x)
+    """A new (n, 3) result like the contiguous positions x, a plain tensor also where x is of a
+    subclass."""
+    return torch.empty_like(x if type(x) is torch.Tensor else x.as_subclass(torch.Tensor))
 
 
 def selfinduced_velocity(positions, strengths, radii, precision="fp64", uniform_core=False):
