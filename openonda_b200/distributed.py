@@ -181,20 +181,21 @@ class ShardedVelocityStretching:
             nt, npairs, per_launch, nv, wsb, (t0, t1, p0, p1) = self.pairs
             self.both_sides = True
             self.ws_bytes = wsb
+            self.ws = torch.empty(max(wsb, 256), dtype=torch.uint8, device=dev)
             self.rows = torch.empty((self.n, nv), dtype=torch.float64, device=dev)
             launches = -(-(p1 - p0) // per_launch)
             # zero, diagonal tiles, diagonal-pair launches, rows, finalize (+ pack)
             self.sweep_launches = 1 + (1 if t1 > t0 else 0) + launches + 2
         else:
-            self.ws_bytes = kernels.workspace_bytes("velocity_and_strength_gradients",
-                                                    precision, self.m, self.n)
+            # (the compact plan's, and its code, where the plain plan's is not free)
+            _, self.ws_bytes, self.sweep_code, self.ws = kernels._scratch(
+                "velocity_and_strength_gradients", self.pcode, self.m, self.n, dev)
             # the sweep's own launches (one-sided: sweep + finalize; both-sides sweep over all
             # particles: zero, diagonal tiles, diagonal-pair launches, finalize); the one launch
             # of small sums reads arrays, not records
             self.sweep_launches = max(2, int(lib.vpm_sweep_launches(
-                _lib.OPS["velocity_and_strength_gradients"], self.pcode, self.m, self.n)))
+                _lib.OPS["velocity_and_strength_gradients"], self.sweep_code, self.m, self.n)))
             self.both_sides = self.sweep_launches > 2
-        self.ws = torch.empty(max(self.ws_bytes, 256), dtype=torch.uint8, device=dev)
         self.kernel_launches_per_call = 1 + self.sweep_launches  # + the pack
 
     def _pair_plan(self, lib):
@@ -223,7 +224,7 @@ class ShardedVelocityStretching:
             return self._sweep_pairs(records)
         _lib.check(_lib.load().vpm_sweep_records(
             _lib.OPS["velocity_and_strength_gradients"], records.data_ptr(), self.n, self.start,
-            self.m, 0, self.u.data_ptr(), self.g.data_ptr(), self.pcode, self.ws.data_ptr(),
+            self.m, 0, self.u.data_ptr(), self.g.data_ptr(), self.sweep_code, self.ws.data_ptr(),
             self.ws.numel(), kernels._stream(self.device)))
         return self.u, self.g
 

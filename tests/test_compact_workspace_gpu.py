@@ -78,3 +78,30 @@ def test_bytes_of_the_fp64_scalars(op):
         records = 64 * n
         assert records < _bytes(op, 0, n) <= records + 16 * 256 * -(-n // 128) + 512, n
         assert _bytes(op, 0, n) <= records + (n << 3) + (1 << 20), n
+
+
+def test_sharded_sweep_in_little_memory():
+    """The sweep of one rank keeps its scratch: the compact plan's where the plain one's is not
+    free."""
+    from openonda_b200 import _lib, kernels
+    from openonda_b200.distributed import ShardedVelocityStretching
+
+    n = 60000
+    x, a, s, *_ = _field(n, 5)
+    want = kernels.velocity_and_strength_gradients(x, a, s)
+    op = "velocity_and_strength_gradients"
+    plain, small = _bytes(op, 0, n), _bytes(op, _lib.COMPACT_WORKSPACE, n)
+    assert small + (64 << 20) < plain
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction(
+        (torch.cuda.memory_reserved() + small + (64 << 20)) / total)
+    try:
+        sweep = ShardedVelocityStretching(n, precision="fp64")
+        assert sweep.ws_bytes == small and sweep.both_sides
+        got = [t.clone() for t in sweep(x, a, s)]
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for g, w in zip(got, want):
+        assert normwise(g.cpu().numpy(), w.cpu().numpy()) <= 1e-12
