@@ -26,13 +26,14 @@ import torch
 from . import _lib
 
 _F64 = torch.float64
+_Tensor = torch.Tensor
 
 
 def _check_vec(name, t, n=None):
-    if (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is _F64 and t.dim() == 2
+    if (isinstance(t, _Tensor) and t.is_cuda and t.dtype is _F64 and t.dim() == 2
             and t.shape[1] == 3 and (n is None or t.shape[0] == n)):
         return t.contiguous()
-    if not isinstance(t, torch.Tensor):
+    if not isinstance(t, _Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if t.device.type != "cuda":
         raise ValueError(f"{name} must be a CUDA tensor (got {t.device})")
@@ -46,10 +47,10 @@ def _check_vec(name, t, n=None):
 
 
 def _check_scalar(name, t, n):
-    if (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is _F64 and t.dim() == 1
+    if (isinstance(t, _Tensor) and t.is_cuda and t.dtype is _F64 and t.dim() == 1
             and t.shape[0] == n):
         return t.contiguous()
-    if not isinstance(t, torch.Tensor):
+    if not isinstance(t, _Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if t.device.type != "cuda":
         raise ValueError(f"{name} must be a CUDA tensor (got {t.device})")
@@ -135,7 +136,7 @@ def _self_inputs(positions, strengths, radii):
 def _out(x):
     """A new (n, 3) result like the contiguous positions x, a plain tensor also where x is of a
     subclass."""
-    return torch.empty_like(x if type(x) is torch.Tensor else x.as_subclass(torch.Tensor))
+    return torch.empty_like(x if type(x) is _Tensor else x.as_subclass(_Tensor))
 
 
 def selfinduced_velocity(positions, strengths, radii, precision="fp64", uniform_core=False):
