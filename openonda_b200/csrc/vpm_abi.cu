@@ -1002,8 +1002,12 @@ struct SetsFinalizeKeGrad {
 // ---- both-sides sweep over a triangle of tile pairs (vpm_triangle.cuh, vpm_circle.cuh) --------
 // Its partial sums may take this much; past it the sweep is the many-launch one (vpm_rot.cuh),
 // whose accumulators do not grow with n^2.  In FP32c the many-launch sweep's waves are long enough
-// from about 150000 particles: velocity 1844 -> 1860 Gpairs/s with the triangle at 140000, 1876 ->
-// 1868 at 200000, 1896 -> 1873 at 330000, fused 963 -> 991 at 140000 and 991 -> 990 at 262144.
+// from about 150000 particles for the velocity with general cores (ms, many launches / triangle):
+// 12.16 / 12.12 at 149999, 13.77 / 13.80 at 160000, 17.30 / 17.43 at 180001, 24.58 / 24.79 at 215000.
+// Above that the others are within 1 % either way but for the fused sum at 160000 (26.33 / 25.83,
+// with one core 25.13 / 24.58; 32.62 / 32.68 at 180001) and the velocity with one core (12.47 / 12.26
+// at 160000, 19.37 / 19.11 at 200000).  LES sums and adjoints are past the 2 GB before 150000 (from
+// about 135000, 129000 and with PSE 83000), the fused sum from about 197000.
 constexpr size_t kMaxTriangleBytes = size_t(2) << 30;
 constexpr int64_t kMaxTriangleN32 = 150000;
 
@@ -1310,7 +1314,7 @@ struct SmallSweep {
         S = s;
         a.windows_per_warp = int(per);
       }
-  }
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(tiles * S));
     cfg.blockDim = dim3(kSmallThreads);

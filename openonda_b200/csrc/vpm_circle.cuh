@@ -22,15 +22,19 @@
 // A target past n (in the last tile) is a particle far away without strength, as a source past n
 // is: the pair's terms underflow to zero on both sides.
 //
-// Memory: nt / 2 sets and a few more of NV values per particle (at n = 16384 and T = 512 about 25
-// sets, 30 MB for the fused sum), written and read once: about 1 % of the sweep.
+// Memory: nt / 2 sets of source sums, and as many sets of target sums as blocks share one list (the
+// small shares of the last lists: up to 128 below about 16384 particles, though most tiles write
+// a few of them).  The fused sum asks for 81 MB at 8192 particles (136 sets), 171 MB at 16384 (144);
+// the adjoint for 3970 MB at 131072.  Written and read once: about 1 % of the sweep.  Past 4 GB
+// (stretching from about 297000 particles, adjoint 137000, with PSE 120000) the sums take several
+// launches (vpm_rot.cuh).
 //
 // Bound: the FP64 pipe at 8 warps per SM (58 operations per unordered pair of the fused sum, root
 // included).  Measured against the one-sided sweeps (us, velocity / fused / stretching / PSE /
 // LES / adjoint / with PSE): 153 / 234 / 220 / 138 / 440 / 550 / 699 -> 109 / 182 / 139 / 91 / 282
 // / 389 / 570 at 8192 particles, 549 / 780 / 744 / 515 / 1555 / 2032 / 2599 -> 375 / 627 / 476 /
-// 305 / 1060 / 1425 / 2114 at 16384; stretching and adjoint at 131072 44.6 / 122.7 / 157.7 -> 28.8
-// / 86.2 / 125.9 ms.
+// 305 / 1060 / 1425 / 2114 at 16384; stretching and adjoint at 131072 44.6 / 122.7 -> 28.8 / 86.2
+// ms (with PSE, in several launches there, 157.7 -> 125.9).
 #pragma once
 
 #include "vpm_rot.cuh"

@@ -5,8 +5,8 @@
 // order; only FP64 additions are ordered differently.  The schedule is the one of
 // vpm_circle.cuh: that kernel launches diagonals one after another, each launch ending in a
 // partly filled wave, while here the tile pairs (I, J), J > I, of all I one after another are cut
-// into shares (vpm_shares.cuh), one block each.  The unit is two batches (64 sources), the span of the longest target window, so that windows start where they
-// do in a tile pair of its own.
+// into shares (vpm_shares.cuh), one block each.  The unit is two batches (64 sources), the span of
+// the longest target window, so that windows start where they do in a tile pair of its own.
 //
 // Source sums of tile I's list go to a set of their own for the particles after tile I, a block's
 // target sums to the set of its place among the blocks that share the list: every element is
@@ -15,7 +15,7 @@
 // Memory: about nt / 2 sets of NV values per particle (at n = 65536 and T = 768, 240 MB for the
 // fused sum), written and read once.
 //
-// Bound: the FP32 pipe, as rot_sweep_kernel.  Measured against its launches (Gpairs/s at 32768 /
+// Bound: the FP32 pipe, as rot_sweep_kernel.  Measured against the launches of its first form (Gpairs/s at 32768 /
 // 65536 / 131072 particles): velocity 1531 / 1685 / 1860 -> 1750 / 1821 / 1858, PSE 1882 / 2078 /
 // 2322 -> 2167 / 2272 / 2331, fused 827 / 935 / 962 -> 892 / 972 / 989, LES 583 / 616 / 627 -> 611
 // / 634 / 642, adjoint 393 / 413 / 421 -> 409 / 423 / 421, with PSE 272 / 278 / 279 -> 279 / 283 /
